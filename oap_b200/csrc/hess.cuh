@@ -40,26 +40,11 @@
 #pragma once
 
 #include "common.cuh"
+#include "devstate.cuh"
 
 namespace oapb {
 
 constexpr int kMaxM = 256;
-
-struct DevState {
-  double fnorm2;    // ||f||^2 of the current residual vector
-  double hnorm2;
-  int dgks;         // second Gram-Schmidt pass needed for the current column
-  int converged;
-  int status;       // bit 0: breakdown (||f|| = 0), bit 1: Schur sweep limit, bit 2: ||f|| not finite
-  int dgks_count;
-  int brk;          // the current basis vector replaces a zero residual (H[j][j-1] = 0)
-  int brk_count;
-  double scale;     // max |theta| over the wanted set
-  double maxest;    // max relative Ritz estimate of the wanted set
-  cplx beta_hat;    // H[k][k-1] after the shifts
-  cplx sigma;       // Q[m-1][k-1]
-  int symtri;       // eigensolves that took the Hermitian tridiagonal path
-};
 
 struct HessArgs {
   const cplx* Hin;  // m x m column-major input

@@ -11,7 +11,9 @@
 //   A32    FP32 copy of the dense operator (mixed form), reference layout
 //   H, Q   m x m complex, column-major; partial-sum buffers of the Gram-Schmidt
 //
-// One Arnoldi step j (executeArnoldiFactorization, ArnoldiProcedures.cpp:407-461):
+// Dense FP64 operators that fit run the steps of a cycle in one launch
+// (cycle.cu).  Elsewhere one Arnoldi step j (executeArnoldiFactorization,
+// ArnoldiProcedures.cpp:407-461) is a chain of kernels:
 //   k_normalize   v_j = f / ||f||, H[j][j-1] = ||f||          (no host sync)
 //   matvec        w = A v_j                                  (HBM-bound)
 //   k_gs_project  partial V^H w per row chunk
@@ -41,6 +43,7 @@
 #include "blocki8.cuh"
 #include "blocktc.cuh"
 #include "common.cuh"
+#include "cycle.cuh"
 #include "gramop.cuh"
 #include "hess.cuh"
 #include "matio.cuh"
@@ -471,6 +474,11 @@ struct oapb_arnoldi {
   int* order = nullptr;
   DevState* st = nullptr;
   int nchunk = 0, chunk = 0, nupd = 0;
+  // one-launch restart cycles (dense operators that fit, cycle.cuh)
+  bool have_cycle = false;
+  CyclePlan cyc;
+  cplx* cpart = nullptr;
+  unsigned* cbar = nullptr;
   // block (multi-vector) buffers: X, W, R, E of up to kBmMaxB vectors each
   static constexpr int kBlocks = 6;
   double *Bre[kBlocks] = {}, *Bim[kBlocks] = {};
@@ -726,18 +734,64 @@ int read_state(oapb_arnoldi* a, DevState* h) {
   return OAPB_OK;
 }
 
+// Whether the FP64 restart loop of the current operator runs as one launch
+// per cycle.  The per-step kernels stay for callbacks and Gram operators
+// (their application is a call or several launches), for operators whose
+// vector does not fit a CTA's shared memory (n above about 10000 complex /
+// 20000 real, where the operator pass takes 90 % of a step), and where a
+// caller asks for the launches themselves: a forced variant of the operator
+// pass or the event timing of every pass.
+bool use_cycle(const oapb_arnoldi* a) {
+  return a->have_cycle && !a->cb && !a->gX && !a->gS && a->a64re && !a->cfg.profile && a->cfg.autotune < 2;
+}
+
+// Two cooperative grids that each held part of the SMs would wait for one
+// another's CTAs: the restart loops of one process take turns.
+std::mutex g_cycle_mu;
+
+// Steps start .. m - 1 in one launch; with `restarted`, the restart's V <- V Q
+// and f first.
+int cycle(oapb_arnoldi* a, int start, bool restarted) {
+  CycleArgs c;
+  c.are = a->a64re;
+  c.aim = a->is_c ? a->a64im : nullptr;
+  c.vre = a->Vre;
+  c.vim = a->Vim;
+  c.fre = a->fre;
+  c.fim = a->fim;
+  c.H = a->H;
+  c.Q = a->Qs;
+  c.part = a->cpart;
+  c.fpart = a->fpart;
+  c.bar = a->cbar;
+  c.st = a->st;
+  c.n = a->n;
+  c.m = a->m;
+  c.j0 = start;
+  c.restart = restarted ? 1 : 0;
+  c.rho = a->cfg.rho;
+  c.seed = a->cfg.seed * 7919ull + (uint64_t)a->stats.restarts * 1024;
+  ++a->stats.kernel_launches;
+  a->stats.matvecs += (uint32_t)(a->m - start);
+  return launch_cycle(a->cyc, c, a->stream);
+}
+
 // One IRAM run until the Ritz estimates reach `tol` or the restart budget
 // is spent.  Returns OAPB_OK / OAPB_NOT_CONVERGED / error.
 template <bool C>
 int iram(oapb_arnoldi* a, bool fp32, double tol, unsigned max_restarts, int start) {
   DevState hs;
+  const bool one = !fp32 && use_cycle(a);
+  std::unique_lock<std::mutex> turn(g_cycle_mu, std::defer_lock);
+  if (one) turn.lock();
+  bool restarted = false;
   for (unsigned r = 0;; ++r) {
-    for (int j = start; j < a->m; ++j) {
-      int rc = arnoldi_step<C>(a, j, fp32);
-      if (rc) return rc;
-    }
+    int rc = OAPB_OK;
+    if (one && start < a->m) rc = cycle(a, start, restarted);
+    for (int j = start; !one && j < a->m && !rc; ++j) rc = arnoldi_step<C>(a, j, fp32);
+    if (rc) return rc;
     const int do_shift = r < max_restarts;
-    int rc = hess(a, do_shift, tol);
+    rc = hess(a, do_shift, tol);
     if (rc) return rc;
     if ((rc = read_state(a, &hs))) return rc;
     if (hs.status & 4) return OAPB_ERR_NONFINITE;
@@ -747,7 +801,10 @@ int iram(oapb_arnoldi* a, bool fp32, double tol, unsigned max_restarts, int star
     a->stats.symtri = (uint32_t)hs.symtri;
     if (hs.converged) return OAPB_OK;
     if (!do_shift) return OAPB_NOT_CONVERGED;
-    if ((rc = restart<C>(a))) return rc;
+    if (one)
+      restarted = true;
+    else if ((rc = restart<C>(a)))
+      return rc;
     a->stats.restarts++;
     start = a->k;
   }
@@ -1735,7 +1792,7 @@ void free_all(oapb_arnoldi* a) {
   drop_gram_stream(a);
   void* ps[] = {a->own64re, a->own64im, a->hvre, a->hvim, a->a32re, a->a32im, a->Vre, a->Vim, a->Xre, a->Xim, a->fre,
                 a->fim, a->wre, a->wim, a->x32re, a->x32im, a->v0re, a->v0im, a->H, a->Qs, a->ritz,
-                a->Y, a->h, a->s, a->part, a->hws, a->est, a->fpart, a->order, a->st};
+                a->Y, a->h, a->s, a->part, a->hws, a->est, a->fpart, a->order, a->st, a->cpart, a->cbar};
   for (void* p : ps)
     if (p) cudaFree(p);
   void* bs[] = {a->abf, a->xbf, a->tcerr, a->Wp, a->wdm, a->bpart, a->bdone, a->gws, a->G, a->G2, a->Rinv, a->bY, a->bQ, a->bH, a->britz, a->best, a->bnorm, a->border,
@@ -1869,6 +1926,11 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
   rc |= dalloc(&a->fpart, sizeof(double) * (a->nupd > 1024 ? a->nupd : 1024));
   rc |= dalloc(&a->order, sizeof(int) * m);
   rc |= dalloc(&a->st, sizeof(DevState));
+  a->have_cycle = cycle_plan(n, m, C, &a->cyc);
+  if (a->have_cycle) {
+    rc |= dalloc(&a->cpart, sizeof(cplx) * (size_t)(m + 1) * a->cyc.ctas);
+    rc |= dalloc(&a->cbar, sizeof(unsigned));
+  }
   const size_t hb = sizeof(cplx) * hess_ws_cplx(m);
   const size_t hb_block = sizeof(cplx) * hess_ws_cplx(kBmMaxB);  // small_eig of the block methods
   int dev = 0, optin = 0;
@@ -1887,7 +1949,8 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
         cudaFuncSetAttribute(k_hess, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attr) != cudaSuccess)
       rc |= OAPB_ERR_CUDA;
   }
-  const size_t vqb = sizeof(cplx) * (size_t)m * m;
+  // (k_vq takes at most m x (k + 4) coefficients, within the device's limit)
+  const size_t vqb = std::min(sizeof(cplx) * (size_t)m * std::min(m, k + 4), (size_t)optin);
   if (vqb > 48 * 1024) {
     cudaFuncSetAttribute(k_vq<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vqb);
     cudaFuncSetAttribute(k_vq<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vqb);
@@ -2004,7 +2067,7 @@ static int make_mixed(oapb_arnoldi* a) {
 static int tune_operator(oapb_arnoldi* a) {
   if (a->cfg.autotune >= 2 && a->cfg.autotune < 2 + kMvVariants) {  // a forced variant
     a->mv64 = a->mv32 = a->cfg.autotune - 2;
-  } else if (a->cfg.autotune == 1) {
+  } else if (a->cfg.autotune == 1 && !use_cycle(a)) {
     // x: the residual buffers (zeroed), y: the work vector
     if (cudaMemsetAsync(a->fre, 0, sizeof(double) * a->n, a->stream) != cudaSuccess) return OAPB_ERR_CUDA;
     if (a->is_c && cudaMemsetAsync(a->fim, 0, sizeof(double) * a->n, a->stream) != cudaSuccess) return OAPB_ERR_CUDA;
