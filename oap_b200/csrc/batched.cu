@@ -25,6 +25,7 @@
 
 #include "common.cuh"
 #include "hess.cuh"
+#include "symeig.cuh"
 
 namespace oapb {
 
@@ -73,6 +74,7 @@ struct BatchSmem {
   int* ord;
   int* order;
   DevState* st;
+  void* sym;  // sym_eig scratch
 };
 
 __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -85,7 +87,8 @@ __host__ __device__ inline size_t batch_smem_bytes(int nmax, int m) {
   b += 2 * (size_t)hess_ld(m) * m * sizeof(cplx);  // T, Z
   b += 4 * (size_t)(m + 1) * sizeof(cplx); // ritz, h, s, u
   b += 2 * (size_t)(m + 1) * sizeof(double) + 64 * sizeof(double);
-  b += 2 * (size_t)(m + 1) * sizeof(int) + sizeof(DevState) + 16 * 16;
+  b += 2 * (size_t)(m + 1) * sizeof(int) + sizeof(DevState) + 16 * 17;
+  b += sym_scratch_bytes(m);
   return b;
 }
 
@@ -118,6 +121,7 @@ __device__ BatchSmem carve(char* base, int nmax, int m) {
   S.ord = (int*)take(sizeof(int) * (m + 1));
   S.order = (int*)take(sizeof(int) * (m + 1));
   S.st = (DevState*)take(sizeof(DevState));
+  S.sym = take(sym_scratch_bytes(m));
   return S;
 }
 
@@ -263,6 +267,8 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
     S.st->status = 0;
     S.st->converged = 0;
     S.st->symtri = 0;
+    S.st->spike = 0;
+    S.st->nosym = 0;
   }
   __syncthreads();
   int start = 0;
@@ -298,7 +304,12 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
           vji[r] = b;
         }
       }
-      if (tid == 0 && j > 0) S.H[j + (j - 1) * m] = cplx{brk ? 0.0 : beta, 0};
+      if (tid == 0 && j > 0) {
+        if (!(rs > 0 && j == start && S.st->spike))  // else row j of H is already there
+          S.H[j + (j - 1) * m] = cplx{brk ? 0.0 : beta, 0};
+        else if (brk)
+          for (int i = 0; i < j; ++i) S.H[j + i * m] = cplx{0, 0};
+      }
       __syncthreads();
       cta_matvec<C, NT>(P.re, P.im, n, S.xr, S.xi, S.wr, S.wi);
       ++matvecs;
@@ -327,7 +338,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
     const int do_shift = rs < A.max_restarts;
     if (tid == 0) S.st->fnorm2 = fnorm2;
     __syncthreads();
-    if (warp == 0) {
+    {
       HessArgs h;
       h.Hin = S.H;
       h.Hout = S.H;
@@ -348,9 +359,14 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       h.use_beta = 1;
       h.tol = A.tol;
       h.beta = 0;
-      // Q is written only at the end of hess_core: until then it is the
+      // a third of the way from k to m: fewer operator applications (4 of 24
+      // with 4 outlying values: 44 -> 38) for the same number of restarts
+      h.keep = k + (m - k) / 3 < m ? k + (m - k) / 3 : k;
+      h.keep_sym = restart_keep(m, k, true);
+      // a symmetric H on the whole CTA, any other on one warp.  Q is written only at the end of hess_core: until then it is the
       // rotation list and eigenvector scratch (2 m + 2 + m k <= m^2 + 2 m + 2)
-      hess_core(h, S.T, S.Z, S.u, S.key, S.ord, S.Q, lane);
+      const bool sym = sym_eig(h, (double*)S.T, (double*)S.Z, sym_scratch(S.sym, m), tid, NT);
+      if (!sym && warp == 0) hess_core(h, S.T, S.Z, S.u, S.key, S.ord, S.Q, lane);
     }
     __syncthreads();
     if (S.st->status & 2) {
@@ -362,21 +378,22 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       status = OAPB_NOT_CONVERGED;
       break;
     }
-    // V[0..k] <- V Q[:, 0..k] in place (each thread owns whole rows r)
+    // V[0..keep] <- V Q[:, 0..keep] in place (each thread owns whole rows r)
+    const int keep = S.st->keep;
     for (int r = tid; r < n; r += NT) {
       cplx out[kBtMaxM + 1];
-      for (int q = 0; q <= k; ++q) out[q] = cplx{0, 0};
+      for (int q = 0; q <= keep; ++q) out[q] = cplx{0, 0};
       for (int i = 0; i < m; ++i) {
         const cplx v = {Vr[(long)i * n + r], C ? Vi[(long)i * n + r] : 0.0};
-        for (int q = 0; q <= k; ++q) out[q] = out[q] + v * S.Q[i + q * m];
+        for (int q = 0; q <= keep; ++q) out[q] = out[q] + v * S.Q[i + q * m];
       }
-      for (int q = 0; q <= k; ++q) {
+      for (int q = 0; q <= keep; ++q) {
         Vr[(long)q * n + r] = out[q].re;
         if (C) Vi[(long)q * n + r] = out[q].im;
       }
       // f = v_k beta_hat + f sigma (Sorensen)
       const cplx f = {S.fr[r], C ? S.fi[r] : 0.0};
-      const cplx nf = out[k] * S.st->beta_hat + f * S.st->sigma;
+      const cplx nf = out[keep] * S.st->beta_hat + f * S.st->sigma;
       S.fr[r] = nf.re;
       if (C) S.fi[r] = nf.im;
     }
@@ -384,7 +401,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
     for (int r = tid; r < n; r += NT) a2 += S.fr[r] * S.fr[r] + (C ? S.fi[r] * S.fi[r] : 0.0);
     fnorm2 = cta_sum2<NT>(a2, 0, S.red).re;
     ++restarts;
-    start = k;
+    start = keep;
   }
   // Ritz vectors x_q = V y_q (q < k) in place, then FP64 residuals
   double scale = 0;

@@ -427,6 +427,8 @@ struct Cycle {
       }
       __syncthreads();
     }
+    // after a restart on the symmetric path row j0 of H is already there
+    const bool spike = a.restart && a.st->spike;
     double s2 = 0, f2;
     for (int r = tid; r < nr; r += kCyThreads) s2 += S.fr[r] * S.fr[r] + (C ? S.fi[r] * S.fi[r] : 0.0);
     norm_partial(s2);
@@ -470,7 +472,12 @@ struct Cycle {
           a.vim[(long)j * n + r0 + r] = u;
         }
       }
-      if (c0 == 0 && tid == 0 && j > 0) a.H[j + (long)(j - 1) * m] = cplx{brk ? 0.0 : beta, 0};
+      if (c0 == 0 && tid == 0 && j > 0) {
+        if (!(spike && j == a.j0))
+          a.H[j + (long)(j - 1) * m] = cplx{brk ? 0.0 : beta, 0};
+        else if (brk)
+          for (int i = 0; i < j; ++i) a.H[j + (long)i * m] = cplx{0, 0};
+      }
       __syncthreads();
       matvec();
       if (!project(S.wr, S.wi, j + 1, S.h)) return false;

@@ -24,7 +24,7 @@ struct CycleArgs {
   DevState* st;
   int n, m;
   int j0;             // first step
-  int restart;        // 1: V <- V Q[:, :j0], f <- v_j0 beta_hat + f sigma first
+  int restart;        // 1: V <- V Q[:, :j0], f <- (V Q)_j0 beta_hat + f sigma first
   double rho;
   uint64_t seed;      // breakdown vectors: seed + j
 };

@@ -18,7 +18,10 @@ struct DevState {
   double maxest;    // max relative Ritz estimate of the wanted set
   cplx beta_hat;    // H[k][k-1] after the shifts
   cplx sigma;       // Q[m-1][k-1]
-  int symtri;       // eigensolves that took the Hermitian tridiagonal path
+  int symtri;       // eigensolves that took the Hermitian path
+  int keep;         // vectors the last restart keeps (the next cycle's first step)
+  int spike;        // row `keep` of H holds the kept Ritz vectors' coupling to the next basis vector
+  int nosym;        // the basis lost the symmetry: the general path from here on
 };
 
 }  // namespace oapb

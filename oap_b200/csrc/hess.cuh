@@ -8,16 +8,17 @@
 //      |T[i][i-1]| <= eps (|T[i-1][i-1]| + |T[i][i]|)), the restatement of
 //      calculateTriangularHEigens (ArnoldiProcedures.cpp:341-349) with a
 //      shifted, deflating iteration instead of the reference's unshifted
-//      one; for a Hermitian H (a Hermitian or real symmetric operator) the
-//      implicit symmetric tridiagonal QR instead;
+//      one; for a Hermitian H (a Hermitian or real symmetric operator) beyond
+//      the sizes of symeig.cuh the implicit symmetric tridiagonal QR instead;
 //   2. Ritz values = diag(T), sorted by the ArnUtils order
 //      (ArnoldiUtils.cpp:24-50); wanted = first k (getWanted,
 //      ArnoldiProcedures.cpp:381-398);
 //   3. eigenvectors y_q = Z u_q of the wanted values (back substitution on
 //      T) and Ritz estimates beta |e_m^T y_q|;
-//   4. if not converged: exact shifts with the unwanted values
+//   4. if not converged: exact shifts with the values after the first `keep`
 //      (iram_shiftedQRIterations, oapGenericArnoldiApi.h:186-222) on H,
-//      Q accumulating the rotations, H compressed to its leading k x k block.
+//      Q accumulating the rotations, H compressed to its leading keep x keep
+//      block.
 // With `dense` set the input is a general matrix, first reduced to
 // Hessenberg form by Householder reflectors accumulated into Z.  The input
 // is scaled by a power of two (exact) so that the rotations need no
@@ -57,10 +58,20 @@ struct HessArgs {
   DevState* st;
   cplx* gws;        // global workspace (hess_ws_cplx(m)) when shared memory is too small
   int m, k, nvec, which, do_shift, real_shifts, dense, use_beta;
+  int keep = 0;      // vectors a restart keeps (k <= keep < m): general path,
+  int keep_sym = 0;  // symmetric path
   double tol;
   double beta;      // used when use_beta == 0 (dense mode: residual norms come separately)
   const int* skip = nullptr;  // k_hess: when set and *skip != 0, return at once (another solver delivered)
 };
+
+// Vectors a restart keeps on the symmetric path: one guard vector beyond the
+// wanted.  It takes most of what more would give (over 32 operators with 8 of
+// 24 at a spectrum's edge, 7800 applications with none, 5600 with one, 4600
+// with five; more of them also leave a warm start little to save).  On the
+// general path a restart costs as much as 20 - 40 applications (its one-warp
+// Schur form), and more kept vectors mean more restarts: the wanted alone.
+__host__ __device__ inline int restart_keep(int m, int k, bool sym) { return sym && k + 1 < m ? k + 1 : k; }
 
 // leading dimension of the T / Z work arrays (odd)
 __host__ __device__ __forceinline__ int hess_ld(int m) { return m | 1; }
@@ -960,7 +971,7 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
   __syncwarp();
   if (sym) {  // the same exact shifts as implicit symmetric tridiagonal steps
     symtri_load(T, Z, m, ld, sd, se, lane);
-    for (int q = k; q < m; ++q) {
+    for (int q = a.keep; q < m; ++q) {
       const R mu = u[q].re;
       int hb = m - 1;
       while (hb > 0) {
@@ -979,7 +990,7 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
     }
     symtri_store(T, m, ld, sd, se, lane);
   } else {
-    for (int q = k; q < m; ++q) {
+    for (int q = a.keep; q < m; ++q) {
       Cx mu = u[q];
       if (a.real_shifts) mu.im = 0;
       int hb = m - 1;
@@ -994,12 +1005,14 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
   }
   __syncwarp();
   if (lane == 0) {
-    st->beta_hat = isig * cx_to(TT_(k, k - 1));
-    st->sigma = cx_to(ZZ_(m - 1, k - 1));
+    st->beta_hat = isig * cx_to(TT_(a.keep, a.keep - 1));
+    st->sigma = cx_to(ZZ_(m - 1, a.keep - 1));
+    st->keep = a.keep;
+    st->spike = 0;
   }
   for (long i = lane; i < mm; i += 32) {
     const int r = (int)(i % m), c = (int)(i / m);
-    a.Hout[i] = (r < k && c < k) ? isig * cx_to(TT_(r, c)) : cplx{0, 0};
+    a.Hout[i] = (r < a.keep && c < a.keep) ? isig * cx_to(TT_(r, c)) : cplx{0, 0};
     a.Qout[i] = cx_to(ZZ_(r, c));
   }
 }

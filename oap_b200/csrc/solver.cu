@@ -49,6 +49,7 @@
 #include "matio.cuh"
 #include "matvec.cuh"
 #include "streamk.cuh"
+#include "symeig.cuh"
 
 namespace oapb {
 
@@ -133,7 +134,11 @@ __global__ void k_normalize(const double* __restrict__ fre, const double* __rest
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (j > 0) H[j + (long)(j - 1) * m] = cplx{st->brk ? 0.0 : beta, 0};
+    // (after a restart on the symmetric path row j of H is already there)
+    if (j > 0 && !(st->spike && j == st->keep))
+      H[j + (long)(j - 1) * m] = cplx{st->brk ? 0.0 : beta, 0};
+    else if (st->brk)
+      for (int i = 0; i < j; ++i) H[j + (long)i * m] = cplx{0, 0};
     if (!(beta > 0) || isinf(beta)) wst->status |= isfinite(beta) ? 1 : 4;
   }
 }
@@ -527,6 +532,8 @@ struct oapb_arnoldi {
   double* bf16err2 = nullptr;
   double bf16_err = -1;
   size_t hess_smem = 0;
+  size_t sym_smem = 0;     // k_symeig (0: m too large for its shared memory)
+  int* symflag = nullptr;  // device: k_symeig delivered
   oapb_arnoldi_stats stats{};
   std::vector<cudaEvent_t> ev_pool;   // profiling events (pairs)
   size_t ev_used = 0;
@@ -702,16 +709,23 @@ int hess(oapb_arnoldi* a, int do_shift, double tol) {
   h.use_beta = 1;
   h.tol = tol;
   h.beta = 0;
+  h.keep = restart_keep(a->m, a->k, false);
+  h.keep_sym = restart_keep(a->m, a->k, true);
+  if (a->sym_smem) {  // a symmetric H first; k_hess returns at once when it was one
+    ++a->stats.kernel_launches;
+    launch_dependent(k_symeig, dim3(1), dim3(sym_threads(h.m)), a->sym_smem, a->stream, h, a->symflag);
+    h.skip = a->symflag;
+  }
   ++a->stats.kernel_launches;
   launch_dependent(k_hess, dim3(1), dim3(hess_threads(h.m)), a->hess_smem, a->stream, h);
   return launch_check();
 }
 
 template <bool C>
-int restart(oapb_arnoldi* a) {
+int restart(oapb_arnoldi* a, int k) {
   cudaStream_t s = a->stream;
-  const int n = a->n, m = a->m, k = a->k;
-  // X[0..k] = V Q[:, 0..k]
+  const int n = a->n, m = a->m;
+  // X[0..k] = V Q[:, 0..k], k the vectors kept
   const size_t shm = sizeof(cplx) * m * (k + 1);
   ++a->stats.kernel_launches;
   k_vq<C><<<grid_n(n), 256, shm, s>>>(a->Vre, a->Vim, n, m, a->Qs, m, k + 1, a->Xre, a->Xim);
@@ -803,10 +817,10 @@ int iram(oapb_arnoldi* a, bool fp32, double tol, unsigned max_restarts, int star
     if (!do_shift) return OAPB_NOT_CONVERGED;
     if (one)
       restarted = true;
-    else if ((rc = restart<C>(a)))
+    else if ((rc = restart<C>(a, hs.keep)))
       return rc;
     a->stats.restarts++;
-    start = a->k;
+    start = hs.keep;
   }
 }
 
@@ -1792,7 +1806,8 @@ void free_all(oapb_arnoldi* a) {
   drop_gram_stream(a);
   void* ps[] = {a->own64re, a->own64im, a->hvre, a->hvim, a->a32re, a->a32im, a->Vre, a->Vim, a->Xre, a->Xim, a->fre,
                 a->fim, a->wre, a->wim, a->x32re, a->x32im, a->v0re, a->v0im, a->H, a->Qs, a->ritz,
-                a->Y, a->h, a->s, a->part, a->hws, a->est, a->fpart, a->order, a->st, a->cpart, a->cbar};
+                a->Y, a->h, a->s, a->part, a->hws, a->est, a->fpart, a->order, a->st, a->cpart, a->cbar,
+                a->symflag};
   for (void* p : ps)
     if (p) cudaFree(p);
   void* bs[] = {a->abf, a->xbf, a->tcerr, a->Wp, a->wdm, a->bpart, a->bdone, a->gws, a->G, a->G2, a->Rinv, a->bY, a->bQ, a->bH, a->britz, a->best, a->bnorm, a->border,
@@ -1936,6 +1951,13 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (sym_smem_bytes(m) + 1024 <= (size_t)optin) {
+    a->sym_smem = sym_smem_bytes(m);
+    rc |= dalloc(&a->symflag, sizeof(int));
+    if (a->sym_smem > 48 * 1024 &&
+        cudaFuncSetAttribute(k_symeig, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024) != cudaSuccess)
+      rc |= OAPB_ERR_CUDA;
+  }
   const size_t static_smem =
       kMaxM * (sizeof(cplx) + sizeof(double) + sizeof(int)) + sizeof(HessShared<cplx, kHessWarps>) + 1024;
   if (hb + static_smem <= (size_t)optin) {
@@ -1949,8 +1971,8 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
         cudaFuncSetAttribute(k_hess, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attr) != cudaSuccess)
       rc |= OAPB_ERR_CUDA;
   }
-  // (k_vq takes at most m x (k + 4) coefficients, within the device's limit)
-  const size_t vqb = std::min(sizeof(cplx) * (size_t)m * std::min(m, k + 4), (size_t)optin);
+  // (k_vq takes m x (kept vectors + 1) or m x (k + 4) coefficients)
+  const size_t vqb = std::min(sizeof(cplx) * (size_t)m * (size_t)std::min(m, std::max(restart_keep(m, k, false), k + 3) + 1), (size_t)optin);
   if (vqb > 48 * 1024) {
     cudaFuncSetAttribute(k_vq<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vqb);
     cudaFuncSetAttribute(k_vq<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vqb);
