@@ -79,12 +79,18 @@ struct BatchSmem {
 
 __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
+// T or Z of hess_core, A or Z of sym_eig
+__host__ __device__ inline size_t batch_tz_bytes(int m) {
+  const size_t a = (size_t)hess_ld(m) * m * sizeof(cplx), b = sym_matrix(m) * sizeof(double);
+  return align16(a > b ? a : b);
+}
+
 __host__ __device__ inline size_t batch_smem_bytes(int nmax, int m) {
   size_t b = 0;
   b += 6 * (size_t)nmax * sizeof(double);  // x, w, f (re / im)
   b += 3 * (size_t)m * m * sizeof(cplx);   // H, Q, Y
   b += (2 * (size_t)m + 2) * sizeof(cplx); // Q tail: rotation list while Q is hess_core scratch
-  b += 2 * (size_t)hess_ld(m) * m * sizeof(cplx);  // T, Z
+  b += 2 * batch_tz_bytes(m);              // T, Z
   b += 4 * (size_t)(m + 1) * sizeof(cplx); // ritz, h, s, u
   b += 2 * (size_t)(m + 1) * sizeof(double) + 64 * sizeof(double);
   b += 2 * (size_t)(m + 1) * sizeof(int) + sizeof(DevState) + 16 * 17;
@@ -107,8 +113,8 @@ __device__ BatchSmem carve(char* base, int nmax, int m) {
   S.fr = (double*)take(sizeof(double) * nmax);
   S.fi = (double*)take(sizeof(double) * nmax);
   S.H = (cplx*)take(sizeof(cplx) * m * m);
-  S.T = (cplx*)take(sizeof(cplx) * hess_ld(m) * m);
-  S.Z = (cplx*)take(sizeof(cplx) * hess_ld(m) * m);
+  S.T = (cplx*)take(batch_tz_bytes(m));
+  S.Z = (cplx*)take(batch_tz_bytes(m));
   S.Q = (cplx*)take(sizeof(cplx) * ((size_t)m * m + 2 * m + 2));
   S.Y = (cplx*)take(sizeof(cplx) * m * m);
   S.ritz = (cplx*)take(sizeof(cplx) * (m + 1));

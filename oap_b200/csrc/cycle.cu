@@ -39,6 +39,7 @@ constexpr int kCyWarps = kCyThreads / 32;
 constexpr int kCyMaxM = 128;
 constexpr int kCyGroups = 8;  // row groups of the projections
 constexpr int kCyMaxSegs = 8;
+constexpr int kCyPre = 4;  // values of f per thread loaded with the norm's partials
 constexpr uint64_t kCyLimitNs = 2000000000ull;
 
 __device__ __forceinline__ uint64_t now_ns() {
@@ -60,13 +61,13 @@ __device__ __forceinline__ double ld_op1(const double* p) {
 }
 
 // Grid barrier on a counter that only grows during the launch: the k-th
-// barrier waits for k gridDim.x arrivals.  One thread arrives (release) and
-// polls (acquire); returns false when the wait ran out.
+// barrier waits for k gridDim.x arrivals.  One thread arrives (release, which
+// with the CTA barrier before it covers the other threads' writes) and polls
+// (acquire); returns false when the wait ran out.
 __device__ bool grid_bar(unsigned* bar, unsigned& target, int* flag) {
   target += gridDim.x;
   __syncthreads();
   if (threadIdx.x == 0) {
-    __threadfence();
     asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
     unsigned v;
     int ok = 1;
@@ -83,7 +84,6 @@ __device__ bool grid_bar(unsigned* bar, unsigned& target, int* flag) {
         }
       }
     }
-    __threadfence();
     *flag = ok;
   }
   __syncthreads();
@@ -148,6 +148,7 @@ struct Cycle {
   long r0;
   unsigned target = 0;
   int tid, warp, lane;
+  double pr[kCyPre];
 
   // w = A x on the CTA's rows (x in shared memory)
   __device__ void matvec() {
@@ -308,8 +309,17 @@ struct Cycle {
     }
   }
   // ||f||^2 from every CTA's share (after a grid barrier; every warp adds
-  // them in the same order)
+  // them in the same order).  The first values of f this thread will scale
+  // into x are loaded beside them, so one trip to L2 covers both (real
+  // operators: the complex ones have no registers to spare).
   __device__ double norm2() {
+#pragma unroll
+    for (int u = 0; u < (C ? 0 : kCyPre); ++u) {
+      const int i = tid + u * kCyThreads;
+      if (i < n) {
+        pr[u] = __ldcg(a.fre + i);
+      }
+    }
     double t = 0;
     for (int c = lane; c < (int)gridDim.x; c += 32) t += __ldcg(a.fpart + c);
     return warp_sum(t);
@@ -458,7 +468,14 @@ struct Cycle {
         break;
       }
       const double inv = 1.0 / beta;
-      for (int i = tid; i < n; i += kCyThreads) {
+#pragma unroll
+      for (int u = 0; u < (C ? 0 : kCyPre); ++u) {
+        const int i = tid + u * kCyThreads;
+        if (i < n) {
+          S.xr[i] = pr[u] * inv;
+        }
+      }
+      for (int i = tid + (C ? 0 : kCyPre) * kCyThreads; i < n; i += kCyThreads) {
         S.xr[i] = __ldcg(a.fre + i) * inv;
         if (C) S.xi[i] = __ldcg(a.fim + i) * inv;
       }

@@ -703,7 +703,7 @@ int hess(oapb_arnoldi* a, int do_shift, double tol) {
   h.keep_sym = restart_keep(a->m, a->k, true);
   if (a->sym_smem) {  // a symmetric H first; k_hess returns at once when it was one
     ++a->stats.kernel_launches;
-    launch_dependent(k_symeig, dim3(1), dim3(sym_threads(h.m)), a->sym_smem, a->stream, h, a->symflag);
+    launch_dependent(k_symeig, dim3(1), dim3(kSymMaxThreads), a->sym_smem, a->stream, h, a->symflag);
     h.skip = a->symflag;
   }
   ++a->stats.kernel_launches;
