@@ -13,6 +13,7 @@
 #include <stdio.h>
 
 #include "common.cuh"
+#include "gemm.cuh"
 #include "matvec.cuh"
 
 namespace oapb {
@@ -32,29 +33,6 @@ __device__ __forceinline__ cplx ldc(const double* re, const double* im, long i) 
 __device__ __forceinline__ void stc(double* re, double* im, long i, cplx v) {
   if (re) re[i] = v.re;
   if (im) im[i] = v.im;
-}
-
-// ------------------------------------------------------------ GEMM (FP64) --
-// C (M x N) = A (M x K) B (K x N), all row-major, complex via optional planes.
-constexpr int GT = 16;
-__global__ void k_gemm(const double* __restrict__ are, const double* __restrict__ aim,
-                       const double* __restrict__ bre, const double* __restrict__ bim,
-                       double* cre, double* cim, int M, int N, int K) {
-  __shared__ cplx As[GT][GT + 1];
-  __shared__ cplx Bs[GT][GT + 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int row = blockIdx.y * GT + ty, col = blockIdx.x * GT + tx;
-  cplx acc = {0, 0};
-  for (int k0 = 0; k0 < K; k0 += GT) {
-    int ka = k0 + tx, kb = k0 + ty;
-    As[ty][tx] = (row < M && ka < K) ? ldc(are, aim, (long)row * K + ka) : cplx{0, 0};
-    Bs[ty][tx] = (kb < K && col < N) ? ldc(bre, bim, (long)kb * N + col) : cplx{0, 0};
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < GT; ++kk) acc = acc + As[ty][kk] * Bs[kk][tx];
-    __syncthreads();
-  }
-  if (row < M && col < N) stc(cre, cim, (long)row * N + col, acc);
 }
 
 // ------------------------------------------------------------- transpose --
@@ -410,10 +388,7 @@ int oapb_dot_product(const oapb_mat* out, const oapb_mat* a, const oapb_mat* b, 
     OAPB_CUDA_TRY(launch_matvec<double>(RE(a), IM(a), M, K, RE(b), IM(b), WRE(out), WIM(out), s));
     return OAPB_OK;
   }
-  dim3 blk(GT, GT), grd((N + GT - 1) / GT, (M + GT - 1) / GT);
-  k_gemm<<<grd, blk, 0, s>>>(RE(a), IM(a), RE(b), IM(b), WRE(out), WIM(out), M, N, K);
-  OAPB_LAUNCH_CHECK();
-  return OAPB_OK;
+  return launch_gemm(RE(a), IM(a), RE(b), IM(b), WRE(out), WIM(out), M, N, K, s);
 }
 
 static int transpose_impl(const oapb_mat* out, const oapb_mat* in, int conj, void* stream) {
