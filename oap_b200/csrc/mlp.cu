@@ -15,11 +15,23 @@
 //    (oapNeuralHost/oapGenericNeuralApi.h:195-360) over CuProceduresApi ops
 //    (dotProduct, tensorProduct, sum).
 //
-// Every layer product is one kernel: C[M x N] = sum_k A(m, k) B(n, k) with
-// strided BF16 operands (the forward product, the data gradient and the
-// weight gradient differ only in strides), 32 x 32 output tiles, FP32
-// accumulation, optional bias + activation epilogue (the pre-activation
-// kept for SIN, whose derivative needs it) and a BF16 copy of the output.
+// Every layer product is one kernel, k_layer: C[M x N] = sum_k A(m, k) B(n, k)
+// with BF16 operands contiguous in either index (the forward product, the data
+// gradient and the weight gradient differ only in that), FP32 accumulation and
+// the layer's elementwise work as its epilogue (bias and activation; the
+// activation's derivative; the bias gradient beside the weight gradient).
+//
+// The sums run in k order on the FP32 pipe, not on the tensor cores: every
+// product rounds its result to BF16 for the next one, and another summation
+// order moves some of those roundings to the other neighbour, which training
+// then amplifies (a tensor-core version took 139 us per step, but two steps
+// moved the gradients by 1e-3 of their norm; this one gives the bits of the
+// 32 x 32 tile it replaces).  The network is small (a step of
+// 16 - 256 - 256 - 2056 on 256 samples is 0.9 GFLOP), so what bounds it is the
+// chain of launches and the longest K loop: 16-byte loads of rows padded to 8
+// values, operands staged as FP32 once, two stages with the next chunk's loads
+// in flight, smaller tiles where a product has few, launches that overlap
+// their predecessors.
 #include <cuda_bf16.h>
 #include <math.h>
 
@@ -28,6 +40,7 @@
 
 #include "common.cuh"
 #include "matio.cuh"
+#include "streamk.cuh"
 
 namespace oapb {
 
@@ -47,8 +60,11 @@ __global__ void k_param_operators(const double* __restrict__ A0, const double* c
 }
 
 // ------------------------------------------------------------ layer GEMM --
-constexpr int kLT = 32;  // output tile
-constexpr int kLK = 16;  // k chunk
+constexpr int kLK = 32;         // k chunk
+constexpr int kLThreads = 256;  // 16 x 16
+constexpr int kBiasBatch = 32;
+
+__host__ __device__ inline int pad8(int x) { return (x + 7) & ~7; }
 
 // activation of a layer's outputs (oapb_activation) and its derivative from
 // the pre-activation z and the output h
@@ -69,94 +85,217 @@ __device__ __forceinline__ float act_df(float z, float h, int act) {
   }
 }
 
-// C[m][n] (ldc) = sum_k A[m*sam + k*sak] * B[n*sbn + k*sbk]; with EPI:
-// z = C + bias[n] (kept in Z when given), C = act(z)
-template <bool EPI>
-__global__ void __launch_bounds__(256) k_layer_gemm(const __nv_bfloat16* __restrict__ A, long sam, long sak,
-                                                    const __nv_bfloat16* __restrict__ Bm, long sbn, long sbk, int M,
-                                                    int N, int K, const float* __restrict__ bias, int act, float* C,
-                                                    float* Z, __nv_bfloat16* Cb, int ldc) {
-  __shared__ float As[kLK][kLT + 1];
-  __shared__ float Bsm[kLK][kLT + 1];
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 2 x 2 outputs each
-  const int m0 = blockIdx.y * kLT, n0 = blockIdx.x * kLT;
-  float acc[2][2] = {{0, 0}, {0, 0}};
-  for (int k0 = 0; k0 < K; k0 += kLK) {
-    for (int e = threadIdx.x; e < kLK * kLT; e += 256) {
-      const int kk = e / kLT, j = e % kLT;
-      const int m = m0 + j, n = n0 + j, k = k0 + kk;
-      As[kk][j] = (m < M && k < K) ? __bfloat162float(A[m * sam + k * sak]) : 0.f;
-      Bsm[kk][j] = (n < N && k < K) ? __bfloat162float(Bm[n * sbn + k * sbk]) : 0.f;
+// Operand X(r, k) of a product: X[r * ld + k] (K-contiguous) or X[k * ld + r];
+// ld a multiple of 8, the pad of a row zero.
+struct LayerArgs {
+  const __nv_bfloat16 *A, *B;
+  int lda, ldb;
+  int M, N, K, tiles_n, tiles;
+  // outputs, each may be null: C FP32 and Z FP32 (ldc = N), Cb BF16 (ldcb)
+  float* C;
+  float* Z;
+  __nv_bfloat16* Cb;
+  int ldcb;
+  const float* bias;     // mode 1
+  const float *H, *Zin;  // mode 2: outputs and pre-activations of the layer below
+  int act;
+  const float* dZ;       // mode 0: FP32 K x M, its column sums to db
+  float* db;
+};
+
+// 8 values (16 bytes) of a staged chunk: rows r .. of one k (row-contiguous) or
+// k .. of one row, zero outside the operand
+template <int ROWS, bool KC>
+struct LayerStage {
+  static constexpr int kCopies = ROWS * kLK / 8;
+  // copy e of the chunk: (row, k) of its first value
+  __device__ static __forceinline__ void at(int e, int& r, int& k) {
+    if (KC) {
+      r = e % ROWS;
+      k = e / ROWS * 8;
+    } else {
+      r = e % (ROWS / 8) * 8;
+      k = e / (ROWS / 8);
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kLK; ++kk) {
-      const float a0 = As[kk][ty * 2], a1 = As[kk][ty * 2 + 1];
-      const float b0 = Bsm[kk][tx * 2], b1 = Bsm[kk][tx * 2 + 1];
-      acc[0][0] = fmaf(a0, b0, acc[0][0]);
-      acc[0][1] = fmaf(a0, b1, acc[0][1]);
-      acc[1][0] = fmaf(a1, b0, acc[1][0]);
-      acc[1][1] = fmaf(a1, b1, acc[1][1]);
-    }
-    __syncthreads();
   }
+  __device__ static __forceinline__ uint4 load(const __nv_bfloat16* X, int ld, int r0, int rows, int k0, int K, int e) {
+    int r, k;
+    at(e, r, k);
+    r += r0;
+    k += k0;
+    if (r >= rows || k >= K) return make_uint4(0, 0, 0, 0);
+    return *reinterpret_cast<const uint4*>(KC ? X + (long)r * ld + k : X + (long)k * ld + r);
+  }
+  // as FP32 into s[k][ROWS]
+  __device__ static __forceinline__ void put(float* s, int e, const uint4& v) {
+    int r, k;
+    at(e, r, k);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    float f[8];
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i) {
+      f[2 * i] = __uint_as_float(w[i] << 16);
+      f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+    if (KC) {
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int m = m0 + ty * 2 + i, n = n0 + tx * 2 + j;
-      if (m < M && n < N) {
-        float v = acc[i][j];
-        if (EPI) {
-          v += bias[n];
-          if (Z) Z[(long)m * ldc + n] = v;
-          v = act_f(v, act);
-        }
-        if (C) C[(long)m * ldc + n] = v;
-        if (Cb) Cb[(long)m * ldc + n] = __float2bfloat16_rn(v);
+      for (int i = 0; i < 8; ++i) s[(k + i) * ROWS + r] = f[i];
+    } else {
+      *reinterpret_cast<float4*>(s + k * ROWS + r) = make_float4(f[0], f[1], f[2], f[3]);
+      *reinterpret_cast<float4*>(s + k * ROWS + r + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+  }
+};
+
+// db[n] = sum_b dZ[b][n] in order of b, one thread per column
+__device__ __forceinline__ void bias_grad(const float* __restrict__ dZ, int B, int N, int n, float* db) {
+  if (n >= N) return;
+  float s = 0;
+  for (int b0 = 0; b0 < B; b0 += kBiasBatch) {
+    float v[kBiasBatch];
+#pragma unroll
+    for (int u = 0; u < kBiasBatch; ++u) v[u] = b0 + u < B ? dZ[(long)(b0 + u) * N + n] : 0.f;
+#pragma unroll
+    for (int u = 0; u < kBiasBatch; ++u)
+      if (b0 + u < B) s += v[u];
+  }
+  db[n] = s;
+}
+
+// MODE 0: C, and the column sums of dZ on the blocks past the tiles; 1: z = C +
+// bias (kept in Z when given), act(z); 2: C act'(h).  A thread computes TM / 16
+// x 2 outputs of a TM x 32 tile.
+template <int MODE, bool AK, bool BK, int TM>
+__global__ void __launch_bounds__(kLThreads) k_layer(LayerArgs g) {
+  constexpr int TN = 32, RM = TM / 16;
+  using SA = LayerStage<TM, AK>;
+  using SB = LayerStage<TN, BK>;
+  static_assert(SA::kCopies + SB::kCopies <= kLThreads, "one copy per thread");
+  __shared__ __align__(16) float As[2][kLK * TM];
+  __shared__ __align__(16) float Bs[2][kLK * TN];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
+  if (MODE == 0 && (int)blockIdx.x >= g.tiles) {
+    bias_grad(g.dZ, g.K, g.M, ((int)blockIdx.x - g.tiles) * kLThreads + tid, g.db);
+    return;
+  }
+  const int n0 = (blockIdx.x % g.tiles_n) * TN, m0 = (blockIdx.x / g.tiles_n) * TM;
+  const int chunks = (g.K + kLK - 1) / kLK;
+  const bool ld_a = tid < SA::kCopies, ld_b = !ld_a && tid - SA::kCopies < SB::kCopies;
+  auto load = [&](int c) {
+    return ld_a ? SA::load(g.A, g.lda, m0, g.M, c * kLK, g.K, tid)
+                : ld_b ? SB::load(g.B, g.ldb, n0, g.N, c * kLK, g.K, tid - SA::kCopies) : make_uint4(0, 0, 0, 0);
+  };
+  auto put = [&](int st, const uint4& v) {
+    if (ld_a) SA::put(As[st], tid, v);
+    if (ld_b) SB::put(Bs[st], tid - SA::kCopies, v);
+  };
+  float acc[RM][2] = {};
+  put(0, load(0));
+  __syncthreads();
+  for (int c = 0; c < chunks; ++c) {
+    const bool more = c + 1 < chunks;
+    uint4 nx = make_uint4(0, 0, 0, 0);
+    if (more) nx = load(c + 1);
+    const float *a = As[c & 1] + ty * RM, *b = Bs[c & 1] + 2 * tx;
+#pragma unroll
+    for (int k = 0; k < kLK; ++k) {
+      float av[RM];
+      if (RM == 2) {
+        const float2 t = *reinterpret_cast<const float2*>(a + k * TM);
+        av[0] = t.x;
+        av[RM - 1] = t.y;
+      } else {
+        av[0] = a[k * TM];
+      }
+      const float2 bv = *reinterpret_cast<const float2*>(b + k * TN);
+#pragma unroll
+      for (int i = 0; i < RM; ++i) {
+        acc[i][0] = fmaf(av[i], bv.x, acc[i][0]);
+        acc[i][1] = fmaf(av[i], bv.y, acc[i][1]);
       }
     }
+    if (more) put((c + 1) & 1, nx);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int m = m0 + ty * RM + i, n = n0 + tx * 2 + j;
+      if (m >= g.M) continue;
+      if (n >= g.N) {  // the BF16 row's pad
+        if (g.Cb && n < g.ldcb) g.Cb[(long)m * g.ldcb + n] = __float2bfloat16_rn(0.f);
+        continue;
+      }
+      const long at = (long)m * g.N + n;
+      float v = acc[i][j];
+      if (MODE == 1) {
+        v += g.bias[n];
+        if (g.Z) g.Z[at] = v;
+        v = act_f(v, g.act);
+      } else if (MODE == 2) {
+        v *= act_df(g.Zin ? g.Zin[at] : 0.f, g.H[at], g.act);
+      }
+      if (g.C) g.C[at] = v;
+      if (g.Cb) g.Cb[(long)m * g.ldcb + n] = __float2bfloat16_rn(v);
+    }
 }
 
-// dY = (Y - T) / B (FP32, and BF16 for the backward products when given);
-// loss partial sums
-__global__ void k_mse_grad(const float* Y, const float* T, int B, long len, __nv_bfloat16* dYb, float* dYf,
-                           double* loss) {
+// Output layer: dZ = (Y - T) / B times the activation's derivative (FP32, and
+// BF16 with row length ldb), and the loss sum (y - t)^2 / (2 B), one atomic per
+// block
+__global__ void __launch_bounds__(256) k_out_grad(const float* __restrict__ Y, const float* __restrict__ T,
+                                                 const float* __restrict__ Z, int act, int B, int N,
+                                                 __nv_bfloat16* dZb, int ldb, float* dZf, double* loss) {
+  __shared__ double red[8];
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   double s = 0;
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < len; e += (long)gridDim.x * blockDim.x) {
-    const float d = Y[e] - T[e];
+  const long len = (long)B * ldb;
+  for (long x = (long)blockIdx.x * blockDim.x + threadIdx.x; x < len; x += (long)gridDim.x * blockDim.x) {
+    const long b = x / ldb;
+    const int n = (int)(x - b * ldb);
+    if (n >= N) {  // the rows' pad
+      dZb[x] = __float2bfloat16_rn(0.f);
+      continue;
+    }
+    const long e = b * N + n;
+    const float y = Y[e], d = y - T[e];
     s += (double)d * d;
-    const float g = d / (float)B;
-    if (dYb) dYb[e] = __float2bfloat16_rn(g);
-    if (dYf) dYf[e] = g;
+    float g = d / (float)B;
+    if (act != OAPB_ACT_LINEAR) g *= act_df(Z ? Z[e] : 0.f, y, act);
+    dZb[x] = __float2bfloat16_rn(g);
+    dZf[e] = g;
   }
   s = warp_sum(s);
-  if ((threadIdx.x & 31) == 0) atomicAdd(loss, 0.5 * s / B);
-}
-
-// dZ = dH * act'(z) (from the output h, or the pre-activation z for SIN),
-// FP32 and BF16 out
-__global__ void k_act_grad(const float* dH, const float* H, const float* Z, int act, long len,
-                           __nv_bfloat16* dZb, float* dZf) {
-  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < len; e += (long)gridDim.x * blockDim.x) {
-    const float g = dH[e] * act_df(Z ? Z[e] : 0.f, H[e], act);
-    dZb[e] = __float2bfloat16_rn(g);
-    if (dZf) dZf[e] = g;
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double q = 0;
+    for (int w = 0; w < 8; ++w) q += red[w];
+    atomicAdd(loss, 0.5 * q / B);
   }
 }
 
-// db[n] = sum_b dZ[b][n]
-__global__ void k_bias_grad(const float* dZ, int B, int N, float* db) {
-  for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
-    float s = 0;
-    for (int b = 0; b < B; ++b) s += dZ[(long)b * N + n];
-    db[n] = s;
-  }
+// where the layers' weights lie: FP32 masters packed, BF16 copies with padded rows
+struct WeightMap {
+  int nl;
+  long off[9];    // first master of layer l; off[nl] = all weights
+  long boff[8];   // first BF16 value of layer l
+  int in[8];      // row length
+};
+__device__ __forceinline__ long weight_bf16_index(const WeightMap& m, long e) {
+  int l = 0;
+  while (l + 1 < m.nl && e >= m.off[l + 1]) ++l;
+  const long r = e - m.off[l];
+  const int in = m.in[l];
+  return m.boff[l] + (r / in) * pad8(in) + r % in;
 }
 
 // Adam on FP32 masters; BF16 working copy refreshed
 __global__ void k_adam(float* w, const float* g, float* m1, float* m2, long len, float lr, float b1, float b2,
-                       float eps, float c1, float c2, __nv_bfloat16* wb) {
+                       float eps, float c1, float c2, __nv_bfloat16* wb, WeightMap map) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < len; e += (long)gridDim.x * blockDim.x) {
     const float gg = g[e];
     const float a = b1 * m1[e] + (1.f - b1) * gg;
@@ -165,13 +304,20 @@ __global__ void k_adam(float* w, const float* g, float* m1, float* m2, long len,
     m2[e] = v;
     const float nw = w[e] - lr * (a / c1) / (sqrtf(v / c2) + eps);
     w[e] = nw;
-    if (wb) wb[e] = __float2bfloat16_rn(nw);
+    if (e < map.off[map.nl]) wb[weight_bf16_index(map, e)] = __float2bfloat16_rn(nw);
   }
 }
 
-__global__ void k_to_bf16(const float* x, long len, __nv_bfloat16* y) {
+// the BF16 copies of all weights
+__global__ void k_weights_bf16(const float* w, __nv_bfloat16* wb, WeightMap map) {
+  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < map.off[map.nl]; e += (long)gridDim.x * blockDim.x)
+    wb[weight_bf16_index(map, e)] = __float2bfloat16_rn(w[e]);
+}
+
+// rows of n values to BF16 rows of ld
+__global__ void k_rows_bf16(const float* __restrict__ x, int n, long len, int ld, __nv_bfloat16* y) {
   for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < len; e += (long)gridDim.x * blockDim.x)
-    y[e] = __float2bfloat16_rn(x[e]);
+    y[(e / n) * ld + e % n] = __float2bfloat16_rn(x[e]);
 }
 
 __global__ void k_init_uniform(float* w, long len, float scale, uint64_t seed) {
@@ -189,16 +335,17 @@ struct oapb_mlp {
   std::vector<long> woff, boff;
   long nparam = 0;
   float *w = nullptr, *g = nullptr, *m1 = nullptr, *m2 = nullptr;  // FP32 [all weights | all biases]
-  __nv_bfloat16* wb = nullptr;                                     // BF16 copy of the weights
+  __nv_bfloat16* wb = nullptr;                                     // BF16 copies of the weights (rows padded)
+  WeightMap map{};
   int step = 0;
   std::vector<int> act;                // activation of each layer's outputs (oapb_activation)
   // activations for the last forward (capacity batch)
   int cap = 0;
   std::vector<float*> hf;              // FP32 activations per layer output (nl)
   std::vector<float*> zf;              // FP32 pre-activations per layer output (nl)
-  std::vector<__nv_bfloat16*> hb;      // BF16 activations: input + per layer
-  float *dA = nullptr, *dB2 = nullptr; // FP32 gradient scratch (cap x max size)
-  __nv_bfloat16 *dAb = nullptr;
+  std::vector<__nv_bfloat16*> hb;      // BF16 activations: input + per layer (rows padded)
+  float* dA[2] = {nullptr, nullptr};   // FP32 dZ of two layers in turn (cap x max size)
+  __nv_bfloat16* dAb[2] = {nullptr, nullptr};  // BF16, rows padded
   double* loss = nullptr;
 };
 
@@ -211,60 +358,88 @@ int g_mlp_free_acts(oapb_mlp* h) {
   h->hf.clear();
   h->hb.clear();
   h->zf.clear();
-  if (h->dA) cudaFree(h->dA);
-  if (h->dB2) cudaFree(h->dB2);
-  if (h->dAb) cudaFree(h->dAb);
-  h->dA = h->dB2 = nullptr;
-  h->dAb = nullptr;
+  for (int i = 0; i < 2; ++i) {
+    if (h->dA[i]) cudaFree(h->dA[i]);
+    if (h->dAb[i]) cudaFree(h->dAb[i]);
+    h->dA[i] = nullptr;
+    h->dAb[i] = nullptr;
+  }
   h->cap = 0;
   return OAPB_OK;
 }
 
-int ensure_acts(oapb_mlp* h, int batch) {
+// zeroed (the row pads stay zero)
+template <typename P>
+int zalloc(P** p, size_t bytes, cudaStream_t s) {
+  if (cudaMalloc(p, bytes) != cudaSuccess) {
+    *p = nullptr;
+    cudaGetLastError();
+    return OAPB_ERR_NOMEM;
+  }
+  return cudaMemsetAsync(*p, 0, bytes, s) == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
+}
+
+int ensure_acts(oapb_mlp* h, int batch, cudaStream_t s) {
   if (batch <= h->cap) return OAPB_OK;
   g_mlp_free_acts(h);
   int mx = 0;
-  for (int s : h->sz) mx = s > mx ? s : mx;
+  for (int v : h->sz) mx = v > mx ? v : mx;
   h->hb.resize(h->nl + 1, nullptr);
   h->hf.resize(h->nl, nullptr);
   h->zf.resize(h->nl, nullptr);
-  for (int l = 0; l <= h->nl; ++l)
-    if (cudaMalloc(&h->hb[l], sizeof(__nv_bfloat16) * (size_t)batch * h->sz[l]) != cudaSuccess) return OAPB_ERR_NOMEM;
-  for (int l = 0; l < h->nl; ++l)
-    if (cudaMalloc(&h->hf[l], sizeof(float) * (size_t)batch * h->sz[l + 1]) != cudaSuccess ||
-        cudaMalloc(&h->zf[l], sizeof(float) * (size_t)batch * h->sz[l + 1]) != cudaSuccess)
-      return OAPB_ERR_NOMEM;
-  if (cudaMalloc(&h->dA, sizeof(float) * (size_t)batch * mx) != cudaSuccess ||
-      cudaMalloc(&h->dB2, sizeof(float) * (size_t)batch * mx) != cudaSuccess ||
-      cudaMalloc(&h->dAb, sizeof(__nv_bfloat16) * (size_t)batch * mx) != cudaSuccess)
-    return OAPB_ERR_NOMEM;
+  int rc = OAPB_OK;
+  for (int l = 0; l <= h->nl && !rc; ++l)
+    rc = zalloc(&h->hb[l], sizeof(__nv_bfloat16) * (size_t)batch * pad8(h->sz[l]), s);
+  for (int l = 0; l < h->nl && !rc; ++l) {
+    rc = zalloc(&h->hf[l], sizeof(float) * (size_t)batch * h->sz[l + 1], s);
+    if (!rc) rc = zalloc(&h->zf[l], sizeof(float) * (size_t)batch * h->sz[l + 1], s);
+  }
+  for (int i = 0; i < 2 && !rc; ++i) {
+    rc = zalloc(&h->dA[i], sizeof(float) * (size_t)batch * mx, s);
+    if (!rc) rc = zalloc(&h->dAb[i], sizeof(__nv_bfloat16) * (size_t)batch * pad8(mx), s);
+  }
+  if (rc) return rc;
   h->cap = batch;
   return OAPB_OK;
 }
 
-void layer_gemm(bool epi, int act, const __nv_bfloat16* A, long sam, long sak, const __nv_bfloat16* Bm, long sbn,
-                long sbk, int M, int N, int K, const float* bias, float* C, float* Z, __nv_bfloat16* Cb, int ldc,
-                cudaStream_t s) {
-  dim3 grid((N + kLT - 1) / kLT, (M + kLT - 1) / kLT);
-  if (epi)
-    k_layer_gemm<true><<<grid, 256, 0, s>>>(A, sam, sak, Bm, sbn, sbk, M, N, K, bias, act, C, Z, Cb, ldc);
-  else
-    k_layer_gemm<false><<<grid, 256, 0, s>>>(A, sam, sak, Bm, sbn, sbk, M, N, K, bias, act, C, Z, Cb, ldc);
+template <int MODE, bool AK, bool BK>
+int layer(LayerArgs g, cudaStream_t s) {
+  // 32 x 32 tiles, 16 x 32 where those leave SMs idle
+  const int tn = (g.N + 31) / 32, tall = tn * ((g.M + 31) / 32);
+  const int tm = tall >= kNumSMs ? 32 : 16;
+  g.tiles_n = tn;
+  g.tiles = tn * ((g.M + tm - 1) / tm);
+  const int extra = MODE == 0 ? (g.M + kLThreads - 1) / kLThreads : 0;
+  const cudaError_t e =
+      tm == 32 ? launch_dependent(k_layer<MODE, AK, BK, 32>, dim3(g.tiles + extra), dim3(kLThreads), 0, s, g)
+               : launch_dependent(k_layer<MODE, AK, BK, 16>, dim3(g.tiles + extra), dim3(kLThreads), 0, s, g);
+  return e == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
 }
 
 int forward_impl(oapb_mlp* h, const float* x, int B, cudaStream_t s) {
-  int rc = ensure_acts(h, B);
+  int rc = ensure_acts(h, B, s);
   if (rc) return rc;
   const long n0 = (long)B * h->sz[0];
-  k_to_bf16<<<grid_for(n0, 256), 256, 0, s>>>(x, n0, h->hb[0]);
-  for (int l = 0; l < h->nl; ++l) {
+  k_rows_bf16<<<grid_for(n0, 256), 256, 0, s>>>(x, h->sz[0], n0, pad8(h->sz[0]), h->hb[0]);
+  for (int l = 0; l < h->nl && !rc; ++l) {
     const int in = h->sz[l], out = h->sz[l + 1];
-    const __nv_bfloat16* W = h->wb + h->woff[l];
-    const float* bias = h->w + h->boff[l];
-    layer_gemm(true, h->act[l], h->hb[l], in, 1, W, in, 1, B, out, in, bias, h->hf[l],
-               h->act[l] == OAPB_ACT_SIN ? h->zf[l] : nullptr, h->hb[l + 1], out, s);
+    LayerArgs g{};
+    g.A = h->hb[l];
+    g.B = h->wb + h->map.boff[l];
+    g.lda = g.ldb = pad8(in);
+    g.M = B;
+    g.N = out;
+    g.K = in;
+    g.C = h->hf[l];
+    g.Z = h->act[l] == OAPB_ACT_SIN ? h->zf[l] : nullptr;
+    g.Cb = h->hb[l + 1];
+    g.ldcb = pad8(out);
+    g.bias = h->w + h->boff[l];
+    g.act = h->act[l];
+    rc = layer<1, true, true>(g, s);
   }
-  return cudaGetLastError() == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
+  return rc ? rc : (cudaGetLastError() == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA);
 }
 
 }  // namespace
@@ -312,12 +487,21 @@ int oapb_mlp_create(oapb_mlp** out, const uint32_t* sizes, uint32_t nlayers, uin
     off += h->sz[l + 1];
   }
   h->nparam = off;
+  long nb = 0;
+  h->map.nl = h->nl;
+  for (int l = 0; l < h->nl; ++l) {
+    h->map.off[l] = h->woff[l];
+    h->map.boff[l] = nb;
+    h->map.in[l] = h->sz[l];
+    nb += (long)pad8(h->sz[l]) * h->sz[l + 1];
+  }
+  h->map.off[h->nl] = nw;
   h->act.assign(h->nl, OAPB_ACT_TANH);
   h->act[h->nl - 1] = OAPB_ACT_LINEAR;
   const size_t fb = sizeof(float) * (size_t)off;
   if (cudaMalloc(&h->w, fb) != cudaSuccess || cudaMalloc(&h->g, fb) != cudaSuccess ||
       cudaMalloc(&h->m1, fb) != cudaSuccess || cudaMalloc(&h->m2, fb) != cudaSuccess ||
-      cudaMalloc(&h->wb, sizeof(__nv_bfloat16) * (size_t)off) != cudaSuccess ||
+      cudaMalloc(&h->wb, sizeof(__nv_bfloat16) * (size_t)nb) != cudaSuccess ||
       cudaMalloc(&h->loss, sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     delete h;
@@ -326,6 +510,7 @@ int oapb_mlp_create(oapb_mlp** out, const uint32_t* sizes, uint32_t nlayers, uin
   cudaMemset(h->m1, 0, fb);
   cudaMemset(h->m2, 0, fb);
   cudaMemset(h->g, 0, fb);
+  cudaMemset(h->wb, 0, sizeof(__nv_bfloat16) * (size_t)nb);
   // uniform(-1/sqrt(fan_in), 1/sqrt(fan_in)) weights, zero biases
   for (int l = 0; l < h->nl; ++l) {
     const long len = (long)h->sz[l] * h->sz[l + 1];
@@ -333,7 +518,7 @@ int oapb_mlp_create(oapb_mlp** out, const uint32_t* sizes, uint32_t nlayers, uin
                                                  seed * 1315423911ull + l);
   }
   cudaMemset(h->w + nw, 0, sizeof(float) * (size_t)(off - nw));
-  k_to_bf16<<<grid_for(off, 256), 256>>>(h->w, off, h->wb);
+  k_weights_bf16<<<grid_for(nw, 256), 256>>>(h->w, h->wb, h->map);
   if (cudaDeviceSynchronize() != cudaSuccess) {
     delete h;
     return OAPB_ERR_CUDA;
@@ -377,33 +562,48 @@ int oapb_mlp_backward(oapb_mlp* h, const float* x, const float* target, uint32_t
   if (!h || !x || !target || batch == 0) return OAPB_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   const int B = (int)batch;
+  if (cudaMemsetAsync(h->loss, 0, sizeof(double), s) != cudaSuccess) return OAPB_ERR_CUDA;
   int rc = forward_impl(h, x, B, s);
   if (rc) return rc;
-  if (cudaMemsetAsync(h->loss, 0, sizeof(double), s) != cudaSuccess) return OAPB_ERR_CUDA;
   const int L = h->nl;
-  const long lenY = (long)B * h->sz[L];
-  // dZ of the output layer into dAb (BF16) / dA (FP32): dY itself for a
-  // linear output, else dY through the activation's derivative
-  if (h->act[L - 1] == OAPB_ACT_LINEAR) {
-    k_mse_grad<<<grid_for(lenY, 256), 256, 0, s>>>(h->hf[L - 1], target, B, lenY, h->dAb, h->dA, h->loss);
-  } else {
-    k_mse_grad<<<grid_for(lenY, 256), 256, 0, s>>>(h->hf[L - 1], target, B, lenY, nullptr, h->dB2, h->loss);
-    k_act_grad<<<grid_for(lenY, 256), 256, 0, s>>>(h->dB2, h->hf[L - 1], h->zf[L - 1], h->act[L - 1], lenY, h->dAb,
-                                                    h->dA);
-  }
+  int cur = 0;  // dZ of the layer at hand
+  launch_dependent(k_out_grad, dim3(grid_for((long)B * pad8(h->sz[L]), 256, kNumSMs * 8)), dim3(256), 0, s,
+                   (const float*)h->hf[L - 1], target, (const float*)h->zf[L - 1], h->act[L - 1], B, h->sz[L],
+                   h->dAb[0], pad8(h->sz[L]), h->dA[0], h->loss);
   for (int l = L - 1; l >= 0; --l) {
     const int in = h->sz[l], out = h->sz[l + 1];
-    // dZ (B x out) in dAb / dA; weight gradient dW[o][i] = sum_b dZ[b][o] X[b][i]
-    layer_gemm(false, 0, h->dAb, 1, out, h->hb[l], 1, in, out, in, B, nullptr, h->g + h->woff[l], nullptr, nullptr,
-               in, s);
-    k_bias_grad<<<grid_for(out, 256), 256, 0, s>>>(h->dA, B, out, h->g + h->boff[l]);
+    // weight gradient dW[o][i] = sum_b dZ[b][o] X[b][i], bias gradient beside it
+    LayerArgs g{};
+    g.A = h->dAb[cur];
+    g.lda = pad8(out);
+    g.B = h->hb[l];
+    g.ldb = pad8(in);
+    g.M = out;
+    g.N = in;
+    g.K = B;
+    g.C = h->g + h->woff[l];
+    g.dZ = h->dA[cur];
+    g.db = h->g + h->boff[l];
+    if ((rc = layer<0, false, false>(g, s))) return rc;
     if (l == 0) break;
-    // data gradient dX[b][i] = sum_o dZ[b][o] W[o][i], then through layer
-    // l - 1's activation
-    const __nv_bfloat16* W = h->wb + h->woff[l];
-    layer_gemm(false, 0, h->dAb, out, 1, W, 1, in, B, in, out, nullptr, h->dB2, nullptr, nullptr, in, s);
-    k_act_grad<<<grid_for((long)B * in, 256), 256, 0, s>>>(h->dB2, h->hf[l - 1], h->zf[l - 1], h->act[l - 1],
-                                                            (long)B * in, h->dAb, h->dA);
+    // data gradient dX[b][i] = sum_o dZ[b][o] W[o][i], through layer l - 1's
+    // activation: dZ of that layer
+    LayerArgs d{};
+    d.A = h->dAb[cur];
+    d.lda = pad8(out);
+    d.B = h->wb + h->map.boff[l];
+    d.ldb = pad8(in);
+    d.M = B;
+    d.N = in;
+    d.K = out;
+    d.C = h->dA[cur ^ 1];
+    d.Cb = h->dAb[cur ^ 1];
+    d.ldcb = pad8(in);
+    d.H = h->hf[l - 1];
+    d.Zin = h->zf[l - 1];
+    d.act = h->act[l - 1];
+    if ((rc = layer<2, true, false>(d, s))) return rc;
+    cur ^= 1;
   }
   if (cudaGetLastError() != cudaSuccess) return OAPB_ERR_CUDA;
   if (loss_out) {
@@ -420,8 +620,8 @@ int oapb_mlp_adam_step(oapb_mlp* h, float lr, void* stream) {
   h->step += 1;
   const float b1 = 0.9f, b2 = 0.999f;
   const float c1 = 1.f - powf(b1, (float)h->step), c2 = 1.f - powf(b2, (float)h->step);
-  k_adam<<<grid_for(h->nparam, 256), 256, 0, s>>>(h->w, h->g, h->m1, h->m2, h->nparam, lr, b1, b2, 1e-8f, c1, c2,
-                                                   h->wb);
+  launch_dependent(k_adam, dim3(grid_for(h->nparam, 256)), dim3(256), 0, s, h->w, (const float*)h->g, h->m1, h->m2,
+                   h->nparam, lr, b1, b2, 1e-8f, c1, c2, h->wb, h->map);
   return cudaGetLastError() == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
 }
 
@@ -441,7 +641,7 @@ int oapb_mlp_set_params(oapb_mlp* h, const float* src, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   if (cudaMemcpyAsync(h->w, src, sizeof(float) * (size_t)h->nparam, cudaMemcpyDefault, s) != cudaSuccess)
     return OAPB_ERR_CUDA;
-  k_to_bf16<<<grid_for(h->nparam, 256), 256, 0, s>>>(h->w, h->nparam, h->wb);
+  k_weights_bf16<<<grid_for(h->nparam, 256), 256, 0, s>>>(h->w, h->wb, h->map);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) return OAPB_ERR_CUDA;
   return OAPB_OK;
 }
