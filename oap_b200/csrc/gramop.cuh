@@ -6,8 +6,7 @@
 
 namespace oapb {
 
-// row splits of the X^T v pass and the partial buffer it needs (doubles)
-int gram_op_splits(int rows, int cols);
+// workspace of launch_gram_apply (doubles)
 size_t gram_op_workspace(int rows, int cols);
 
 // w = X (X^T v) (accumulate: w += X (X^T v)); v, w: rows FP64 values; ws:

@@ -614,11 +614,11 @@ int apply_op(oapb_arnoldi* a, const double* xre, const double* xim, double* yre,
     return rc == 0 ? OAPB_OK : OAPB_ERR_CALLBACK;
   }
   if (a->gX) {
-    a->stats.kernel_launches += 3;
+    a->stats.kernel_launches += 2;
     return launch_gram_apply(a->gX, n, a->gcols, xre, yre, a->gws, s);
   }
   if (a->gS) {
-    a->stats.kernel_launches += 3 * (uint64_t)gram_stream_blocks(a->gS);
+    a->stats.kernel_launches += 2 * (uint64_t)gram_stream_blocks(a->gS);
     return gram_stream_apply(a->gS, xre, yre, s);
   }
   Timed tm{nullptr, nullptr, 0, fp32 ? 1 : 0, 1};
@@ -671,7 +671,12 @@ int arnoldi_step(oapb_arnoldi* a, int j, bool fp32) {
   a->stats.matvecs++;
   if ((rc = gs_pass<C>(a, j, a->wre, a->wim, a->h, 0))) return rc;
   ++a->stats.kernel_launches;
-  k_gs_finalize<<<1, 256, 0, s>>>(a->fpart, a->nupd, a->h, a->s, a->H, m, j, a->cfg.rho, a->st, 0, !C);
+  // A Gram operator's application reads X (hundreds of microseconds at the
+  // sizes it is for), so its vectors are reorthogonalised at every step: the
+  // rho rule leaves 1e-6 of orthogonality on image spectra, and H then fails
+  // the symmetry check (a general eigensolve at m = 96 took 20 ms)
+  const double rho = (a->gX || a->gS) ? 1e300 : a->cfg.rho;
+  k_gs_finalize<<<1, 256, 0, s>>>(a->fpart, a->nupd, a->h, a->s, a->H, m, j, rho, a->st, 0, !C);
   if ((rc = gs_pass<C>(a, j, a->fre, a->fim, a->s, 1))) return rc;
   ++a->stats.kernel_launches;
   k_gs_finalize<<<1, 256, 0, s>>>(a->fpart, a->nupd, a->h, a->s, a->H, m, j, a->cfg.rho, a->st, 1, !C);
