@@ -57,12 +57,14 @@ constexpr uint32_t kI8ATile = kI8M * kI8K;  // bytes of one operator slice tile
 // v = sum_i out[i] 2^-7(i+1) + remainder, |remainder| <= 2^-(7n+1).
 template <int NS>
 __device__ __forceinline__ void slice_value(double v, int (&out)[NS]) {
+  // adding 1.5 2^52 rounds to the nearest integer (ties to even, as rint) and
+  // leaves it in the low word: three operations per slice, no conversion
+  constexpr double kRound = 6755399441055744.0;
 #pragma unroll
   for (int i = 0; i < NS; ++i) {
-    v *= 128.0;
-    const double t = rint(v);
-    out[i] = (int)t;
-    v -= t;
+    const double t = fma(v, 128.0, kRound);
+    out[i] = __double2loint(t);
+    v = fma(v, 128.0, kRound - t);
   }
 }
 
@@ -91,41 +93,78 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
          ((uint32_t)(d & 0xff) << 24);
 }
 
-// One block per operator row: the row scale of both planes, then the 6
-// slices of 4 consecutive columns per thread (one 32-bit store per slice).
+// The mixed form's copies of the operator in one pass over it: a CTA takes the
+// rows blockIdx.x, + gridDim.x, ...; the row scale of both planes first, then
+// the row again (two CTAs of 512 threads per SM keep 296 rows in flight, 77 MB
+// at n = 16384 complex, so the second read comes from L2) for the 6 int8 slices
+// and the BF16 hi / lo planes of 4 consecutive columns per thread, and
+// ||A - hi||_F^2 summed into err2.  HBM bounds it: 8 bytes read and 10 written
+// per element and plane.  The separate passes it replaces (a slice pass with a
+// CTA per row, a BF16 pass per plane) read the operator two to three times:
+// n = 13689 complex 2.9 ms.
+constexpr int kSplitThreads = 512;
+
 template <bool CPLX>
-__global__ void __launch_bounds__(256) k_split_operator_i8(const double* __restrict__ are,
-                                                           const double* __restrict__ aim, int n, int kp, long row0,
-                                                           int8_t* __restrict__ sl, double* __restrict__ rscale) {
-  __shared__ double red[8];
-  const long r = row0 + blockIdx.x;
-  const double* pr = are + r * n;
-  const double* pi = CPLX ? aim + r * n : nullptr;
-  double m = 0.0;
-  for (int c = threadIdx.x; c < n; c += blockDim.x) {
-    m = fmax(m, fabs(pr[c]));
-    if (CPLX) m = fmax(m, fabs(pi[c]));
-  }
-  m = block_max(m, red);
-  const int e = scale_exponent(m);
-  if (threadIdx.x == 0) rscale[r] = ldexp(1.0, e);
-  const double inv = ldexp(1.0, -e);
+__global__ void __launch_bounds__(kSplitThreads, 2)
+    k_split_operator(const double* __restrict__ are, const double* __restrict__ aim, int n, int kp, long row0,
+                     long rows, int8_t* __restrict__ sl, double* __restrict__ rscale, __nv_bfloat16* __restrict__ bf,
+                     double* err2) {
+  __shared__ double red[kSplitThreads / 32];
   const size_t plane = (size_t)n * kp;
-  for (int c4 = threadIdx.x; c4 < kp / 4; c4 += blockDim.x) {
+  double acc = 0;
+  for (long x = blockIdx.x; x < rows; x += gridDim.x) {
+    const long r = row0 + x;
+    double m = 0.0;
 #pragma unroll
     for (int p = 0; p < (CPLX ? 2 : 1); ++p) {
-      const double* src = p == 0 ? pr : pi;
-      int d[4][kI8SlicesA];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int c = 4 * c4 + t;
-        slice_value<kI8SlicesA>(c < n ? src[c] * inv : 0.0, d[t]);
-      }
-#pragma unroll
-      for (int i = 0; i < kI8SlicesA; ++i)
-        *reinterpret_cast<uint32_t*>(sl + (p * kI8SlicesA + i) * plane + (size_t)r * kp + 4 * c4) =
-            pack4(d[0][i], d[1][i], d[2][i], d[3][i]);
+      const double* src = (p == 0 ? are : aim) + r * n;
+#pragma unroll 8
+      for (int c = threadIdx.x; c < n; c += kSplitThreads) m = fmax(m, fabs(src[c]));
     }
+    m = block_max(m, red);
+    const int e = scale_exponent(m);
+    if (threadIdx.x == 0) rscale[r] = ldexp(1.0, e);
+    const double inv = ldexp(1.0, -e);
+#pragma unroll
+    for (int p = 0; p < (CPLX ? 2 : 1); ++p) {
+      const double* src = (p == 0 ? are : aim) + r * n;
+      int8_t* s8 = sl + (size_t)(p * kI8SlicesA) * plane + (size_t)r * kp;
+      __nv_bfloat16* hi = bf + (size_t)(2 * p) * plane + (size_t)r * kp;
+      __nv_bfloat16* lo = hi + plane;
+#pragma unroll 2
+      for (int c4 = threadIdx.x; c4 < kp / 4; c4 += kSplitThreads) {
+        int d[4][kI8SlicesA];
+        alignas(8) __nv_bfloat16 h[4];
+        alignas(8) __nv_bfloat16 l[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int c = 4 * c4 + t;
+          const double ad = c < n ? src[c] : 0.0;
+          slice_value<kI8SlicesA>(ad * inv, d[t]);
+          const float v = (float)ad;
+          h[t] = __float2bfloat16_rn(v);
+          const float hf = __bfloat162float(h[t]);
+          l[t] = __float2bfloat16_rn(v - hf);
+          const double dd = ad - (double)hf;
+          acc = fma(dd, dd, acc);
+        }
+#pragma unroll
+        for (int i = 0; i < kI8SlicesA; ++i)
+          *reinterpret_cast<uint32_t*>(s8 + (size_t)i * plane + 4 * c4) = pack4(d[0][i], d[1][i], d[2][i], d[3][i]);
+        *reinterpret_cast<uint2*>(hi + 4 * c4) = *reinterpret_cast<const uint2*>(h);
+        *reinterpret_cast<uint2*>(lo + 4 * c4) = *reinterpret_cast<const uint2*>(l);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0;
+    for (int w = 0; w < kSplitThreads / 32; ++w) t += red[w];
+    atomicAdd(err2, t);
   }
 }
 
@@ -539,15 +578,15 @@ SkGrid i8_grid(int n, int kp) { return sk_grid((n + kI8M - 1) / kI8M, kp / kI8K,
 
 }  // namespace
 
-int split_operator_i8(const double* are, const double* aim, int n, int kp, int8_t* slices, double* rscale,
-                      cudaStream_t s, long row0, long rows) {
-  if (rows < 0) rows = n - row0;
+int split_operator(const double* are, const double* aim, int n, int kp, int8_t* slices, double* rscale,
+                   __nv_bfloat16* bf, double* err2, cudaStream_t s, long row0, long rows) {
   if (row0 < 0 || row0 + rows > n || kp % 128 || kp < n) return OAPB_ERR_ARG;
   if (rows == 0) return OAPB_OK;
+  const unsigned grid = (unsigned)(rows < 2 * kNumSMs ? rows : 2 * kNumSMs);
   if (aim)
-    k_split_operator_i8<true><<<(unsigned)rows, 256, 0, s>>>(are, aim, n, kp, row0, slices, rscale);
+    k_split_operator<true><<<grid, kSplitThreads, 0, s>>>(are, aim, n, kp, row0, rows, slices, rscale, bf, err2);
   else
-    k_split_operator_i8<false><<<(unsigned)rows, 256, 0, s>>>(are, nullptr, n, kp, row0, slices, rscale);
+    k_split_operator<false><<<grid, kSplitThreads, 0, s>>>(are, nullptr, n, kp, row0, rows, slices, rscale, bf, err2);
   return cudaGetLastError() == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
 }
 

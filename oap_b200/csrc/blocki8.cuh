@@ -2,6 +2,7 @@
 // tensor cores (blocki8.cu).
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -32,10 +33,12 @@ inline size_t i8_block_bytes(int kp) { return (size_t)kI8SlicesX * 64 * kp; }
 constexpr int kI8BlockScales = 64;
 constexpr int kI8ScaleDoubles = kI8BlockScales + 148 * 32;
 
-// Slices of rows row0 .. row0 + rows - 1 (rows < 0: to the last row) of the
-// FP64 operator (aim NULL for a real operator).
-int split_operator_i8(const double* are, const double* aim, int n, int kp, int8_t* slices, double* rscale,
-                      cudaStream_t s, long row0 = 0, long rows = -1);
+// Rows row0 .. row0 + rows - 1 of the FP64 operator (aim NULL for a real one)
+// as int8 slices with their row scales and as BF16 hi / lo planes (bf: re hi,
+// re lo, im hi, im lo, n x kp each); ||A - hi||_F^2 of the rows is added to
+// *err2.
+int split_operator(const double* are, const double* aim, int n, int kp, int8_t* slices, double* rscale,
+                   __nv_bfloat16* bf, double* err2, cudaStream_t s, long row0, long rows);
 
 // Largest b the pass takes (complex / real operator).
 inline int i8_max_vectors(bool cplx) { return cplx ? 16 : 32; }

@@ -1973,7 +1973,6 @@ static int build_tc_planes(oapb_arnoldi* a, long row0, long rows) {
     if (cudaMemsetAsync(a->bf16err2, 0, sizeof(double), a->stream) != cudaSuccess) return OAPB_ERR_CUDA;
     a->bf16_err = -1;
   }
-  a->stats.kernel_launches += np / 2;
   // int8 slices of the FP64-class pass (optional: without the memory the
   // FP64 pass stays on the FP64 tensor cores)
   if (row0 == 0) {
@@ -1989,18 +1988,20 @@ static int build_tc_planes(oapb_arnoldi* a, long row0, long rows) {
       cudaGetLastError();
     }
   }
-  if (a->ai8) {
+  if (a->ai8) {  // both copies in one pass over the operator
     ++a->stats.kernel_launches;
-    if (split_operator_i8(a->a64re, a->is_c ? a->a64im : nullptr, a->n, a->kp, a->ai8, a->ai8s, a->stream, row0,
-                          rows))
+    if (split_operator(a->a64re, a->is_c ? a->a64im : nullptr, a->n, a->kp, a->ai8, a->ai8s, a->abf, a->bf16err2,
+                       a->stream, row0, rows))
       return OAPB_ERR_CUDA;
     a->have_i8 = true;
+  } else {
+    for (int p = 0; p < np / 2; ++p) {
+      ++a->stats.kernel_launches;
+      if (split_operator_bf16(p ? a->a64im : a->a64re, a->n, a->kp, a->abf + 2 * p * plane,
+                              a->abf + (2 * p + 1) * plane, a->stream, row0, rows, a->bf16err2))
+        return OAPB_ERR_CUDA;
+    }
   }
-  if (split_operator_bf16(a->a64re, a->n, a->kp, a->abf, a->abf + plane, a->stream, row0, rows, a->bf16err2))
-    return OAPB_ERR_CUDA;
-  if (a->is_c && split_operator_bf16(a->a64im, a->n, a->kp, a->abf + 2 * plane, a->abf + 3 * plane, a->stream, row0,
-                                     rows, a->bf16err2))
-    return OAPB_ERR_CUDA;
   a->have_tc = true;
   return OAPB_OK;
 }
