@@ -222,7 +222,7 @@ typedef struct oapb_arnoldi_config {
   int32_t tensor_cores;    /* 1 (default): block operator passes on the
                               tensor cores (FP32-class passes as split BF16
                               tcgen05, FP64 passes as DMMA); 0: CUDA cores */
-  int32_t refine;          /* mixed form, complex LM problems: 1 (default)
+  int32_t refine;          /* mixed form, LM problems: 1 (default)
                               refines the FP32-phase subspace by FP64
                               residual + FP32-class Sylvester corrections;
                               0 runs FP64 subspace iteration instead */
