@@ -469,8 +469,9 @@ OAPB_EXPORT int oapb_gram_build(const float* X, uint32_t rows, uint32_t cols,
                                 float* A, double* A64, void* stream);
 /* The build's workspace (BF16 hi / lo planes of X, 4 bytes per element of X,
  * plus the tile partials) comes from a library-owned stream-ordered pool
- * that keeps the memory for the next build; this returns it to the driver
- * (current device; no counterpart in the reference). */
+ * that keeps the memory for the next build, and so does the batched solver's
+ * (up to 1 GiB); this returns it to the driver (current device; no counterpart
+ * in the reference). */
 OAPB_EXPORT int oapb_gram_trim(void);
 
 /* Image ingestion: `count` decoded RGB8 images of `pixels` pixels each
@@ -507,9 +508,10 @@ typedef struct oapb_batch_stats {
   double seconds;        /* host wall time of the call */
   uint32_t variant;      /* launch variant (cfg.autotune: 1 tunes, 2 + v forces v) */
   uint32_t threads;      /* threads per CTA of that variant */
-  uint64_t operator_bytes; /* operator bytes read by all matvecs (8 n^2 real,
-                              16 n^2 complex each): the launch's algorithmic
-                              HBM traffic */
+  uint64_t operator_bytes; /* operator bytes read (8 n^2 real, 16 n^2 complex
+                              per pass; the residual check takes up to three
+                              pairs per pass): the launch's algorithmic HBM
+                              traffic */
 } oapb_batch_stats;
 
 /* Solve `count` independent eigenproblems (IEigenCalculator::calculate,
@@ -520,11 +522,11 @@ typedef struct oapb_batch_stats {
  * hdim <= 32), wanted, sort, tolerance, max_restarts, rho, seed, autotune
  * (0: the default launch variant, 256 threads per CTA; 1: the variant
  * (threads per CTA x CTAs per SM the registers are budgeted for: 256 x 1,
- * 128 x 2, 256 x 2, 128 x 4, 64 x 8) that ran fastest on a sample of the
- * first batch of a given largest n, hdim, wanted and complexity, cached per
- * device; 2 + v: variant v, 0..4); n, is_complex, precision and init are
- * ignored (complex iff im != NULL, FP64, seeded random start).  `problems` is a HOST array.  Host outputs:
- * eig_re / eig_im / residuals (count x wanted, row i = problem i in sort
+ * 128 x 2, 256 x 2, 128 x 4, 64 x 8) of 256 x 2, 128 x 2 and 128 x 4 that ran
+ * fastest on a sample of the first batch of a given largest n, hdim, wanted and
+ * complexity, cached per device; 2 + v: variant v, 0..4); n, is_complex,
+ * precision and init are ignored (complex iff im != NULL, FP64, seeded random
+ * start).  `problems` is a HOST array.  Host outputs: eig_re / eig_im / residuals (count x wanted, row i = problem i in sort
  * order), status (count, oapb_status per problem).  Synchronises `stream`.
  * Returns OAPB_OK when every problem converged, OAPB_NOT_CONVERGED when some
  * did not (see status), or an error. */

@@ -7,17 +7,28 @@
 // (256 threads) pulls the next problem from an atomic queue ordered by
 // decreasing n (largest first, for load balance over uneven sizes) and runs
 // the whole restart loop on the device: Arnoldi steps with CGS + DGKS
-// (rho rule), the one-warp Schur / exact-shift restart (hess_core), the
-// in-place V <- V Q, Sorensen's residual update, Ritz vectors and the FP64
-// residual of every wanted pair.  There are no host round trips between
-// restarts, so no per-restart launch or graph replay exists at all.
+// (rho rule), the restart's small eigenproblem (sym_eig on the whole CTA for a
+// symmetric H, hess_core on one warp for any other), V Q and the residual
+// update, Ritz vectors and the FP64 residual of every wanted pair.  There are
+// no host round trips between restarts, so no per-restart launch or graph
+// replay exists at all.
 //
 // Shared memory per CTA: the current vector x, w and f (n complex each), H,
-// the Schur workspaces T and Z, Q, Y (m x m complex each) and small arrays.
-// The Krylov basis V ((hdim + 1) x n complex) lives in a global workspace
-// slot owned by the CTA (L2-resident).
+// the eigenproblem's workspaces T and Z, Q, Y (m x m complex each) and small
+// arrays.  Two copies of the Krylov basis V ((hdim + 1) x n complex) live in a
+// global workspace slot owned by the CTA (L2-resident): a restart writes V Q
+// from one to the other.
+//
+// What bounds it: the operators' stream from HBM (every application reads its
+// n x n matrix once), and between two applications the serial chain of a
+// step's reductions; two CTAs per SM cover one another's.  2048 complex
+// problems of 32..256 rows, hdim 24, 4 wanted: 43.7 ms with one CTA per SM,
+// V Q through local memory and a pass over the operator per checked pair,
+// 28.4 with 256 x 2, V Q in registers and three pairs per pass.
 #include <algorithm>
 #include <chrono>
+#include <string.h>
+
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -25,6 +36,7 @@
 
 #include "common.cuh"
 #include "hess.cuh"
+#include "pool.cuh"
 #include "symeig.cuh"
 
 namespace oapb {
@@ -56,7 +68,7 @@ struct BatchArgs {
   int mcap, k, which, max_restarts;
   double tol, rho;
   uint64_t seed;
-  double* vws;      // per-CTA basis slots: 2 planes x (mcap + 1) x nmax
+  double* vws;      // per-CTA basis slots: 2 copies x 2 planes x (mcap + 1) x nmax
   int nmax;
   double* ev_re;    // count x k
   double* ev_im;
@@ -64,7 +76,7 @@ struct BatchArgs {
   int* status;      // count
   unsigned long long* matvecs;
   unsigned long long* restarts;
-  unsigned long long* op_bytes;  // operator bytes the matvecs read (8 n^2 real, 16 n^2 complex each)
+  unsigned long long* op_bytes;  // operator bytes read (8 n^2 real, 16 n^2 complex per pass)
 };
 
 struct BatchSmem {
@@ -152,7 +164,6 @@ __device__ __forceinline__ cplx cta_sum2(double a, double b, double* red) {
   return cplx{ra, rb};
 }
 
-// w = A x  (A row-major n x n; warps over rows, lanes over columns)
 // w = A x for one problem (A row-major split planes in global memory, x in
 // shared memory): warp w takes kMvRows rows at a time, the lanes stride the
 // columns; the loads of all its rows are issued together (the operator
@@ -196,6 +207,65 @@ __device__ void cta_matvec(const double* __restrict__ Are, const double* __restr
       }
     }
   }
+}
+
+// Residuals of NV vectors in one pass over A: per vector v the sums over the
+// rows of |(A x_v)_r - lam_v x_v[r]|^2 and |x_v[r]|^2, added up over the CTA.
+// Two rows per warp and pass: the operator streams from HBM, and the NV
+// vectors share its loads (4 wanted pairs: two passes instead of four).
+constexpr int kBtVerify = 3;  // vectors per pass: the x, w and f buffers
+template <bool C, int NT, int NV>
+__device__ void cta_residuals(const double* __restrict__ Are, const double* __restrict__ Aim, int n,
+                              const double* const (&xr)[kBtVerify], const double* const (&xi)[kBtVerify],
+                              const cplx (&lam)[kBtVerify], double* red, cplx (&sums)[kBtVerify]) {
+  constexpr int R = 2;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  double e2[NV], x2[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) e2[v] = x2[v] = 0.0;
+  for (int r0 = R * w; r0 < n; r0 += R * (NT / 32)) {
+    const int nr = n - r0 < R ? n - r0 : R;
+    double sr[R][NV], si[R][NV];
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) sr[q][v] = si[q][v] = 0.0;
+#pragma unroll 4
+    for (int c = l; c < n; c += 32) {
+      double a[R], b[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const long idx = (long)(r0 + (q < nr ? q : 0)) * n + c;
+        a[q] = __ldcs(Are + idx);
+        b[q] = C ? __ldcs(Aim + idx) : 0.0;
+      }
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const double x0 = xr[v][c], x1 = C ? xi[v][c] : 0.0;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          sr[q][v] = fma(a[q], x0, sr[q][v]);
+          if (C) {
+            sr[q][v] = fma(-b[q], x1, sr[q][v]);
+            si[q][v] = fma(a[q], x1, fma(b[q], x0, si[q][v]));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        const double p = warp_sum(sr[q][v]), t = C ? warp_sum(si[q][v]) : 0.0;
+        if (l == 0 && q < nr) {
+          const cplx x = {xr[v][r0 + q], C ? xi[v][r0 + q] : 0.0};
+          e2[v] += abs2(cplx{p, t} - lam[v] * x);
+          x2[v] += abs2(x);
+        }
+      }
+  }
+#pragma unroll
+  for (int v = 0; v < NV; ++v) sums[v] = cta_sum2<NT>(e2[v], x2[v], red);
 }
 
 // coef[i] = sum_r conj(V_i[r]) src[r], i < nvec (warps over vectors)
@@ -247,16 +317,51 @@ __device__ double cta_update(const double* Vr, const double* Vi, int n, int nvec
   return cta_sum2<NT>(s2, 0.0, red).re;
 }
 
+// out[c] = sum_i V_i[r] B[i + (q0 + c) ldb], i < m, for the columns q0 + c < nq.
+// Six complex columns at a time stay in registers at 256 threads x 2 CTAs; row
+// r of V is read again from L2 per six columns.  An array of all m sums in local
+// memory, which an update in place needs, took about a third of the launch.
+constexpr int kBtCols = 6;
+template <bool C>
+__device__ __forceinline__ void cta_combine(const double* Vr, const double* Vi, int n, int r, int m, const cplx* B,
+                                            int ldb, int q0, int nq, cplx (&out)[kBtCols]) {
+  int col[kBtCols];
+#pragma unroll
+  for (int c = 0; c < kBtCols; ++c) {
+    out[c] = cplx{0, 0};
+    col[c] = (q0 + c < nq ? q0 + c : q0) * ldb;
+  }
+#pragma unroll 2
+  for (int i = 0; i < m; ++i) {
+    const double p = Vr[(long)i * n + r], q = C ? Vi[(long)i * n + r] : 0.0;
+#pragma unroll
+    for (int c = 0; c < kBtCols; ++c) {
+      const cplx b = B[i + col[c]];
+      out[c].re = fma(p, b.re, out[c].re);
+      out[c].im = fma(p, b.im, out[c].im);
+      if (C) {
+        out[c].re = fma(-q, b.im, out[c].re);
+        out[c].im = fma(q, b.re, out[c].im);
+      }
+    }
+  }
+}
+
 template <bool C, int NT>
 __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, const BatchSmem& S) {
   const int n = P.n;
   const int m = n < A.mcap ? n : A.mcap;
   const int k = A.k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  double* Vr = A.vws + (size_t)slot * 2 * (A.mcap + 1) * A.nmax;
-  double* Vi = Vr + (size_t)(A.mcap + 1) * A.nmax;
+  // two copies of the basis: a restart (and the Ritz vectors) goes from one to
+  // the other, so its sums stay in registers a few columns at a time
+  const size_t vplane = (size_t)(A.mcap + 1) * A.nmax;
+  double* Vr = A.vws + (size_t)slot * 4 * vplane;
+  double* Vi = Vr + vplane;
+  double* Nr = Vr + 2 * vplane;
+  double* Ni = Vr + 3 * vplane;
   const uint64_t pseed = A.seed * 0x9E3779B97F4A7C15ull + (uint64_t)P.index * 0xD1B54A32D192ED03ull;
-  unsigned long long matvecs = 0, restarts = 0;
+  unsigned long long matvecs = 0, restarts = 0, passes = 0;  // passes over the operator
   int status = OAPB_OK;
   if (m <= k || m < 2) status = OAPB_ERR_ARG;
 
@@ -319,6 +424,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       __syncthreads();
       cta_matvec<C, NT>(P.re, P.im, n, S.xr, S.xi, S.wr, S.wi);
       ++matvecs;
+      ++passes;
       __syncthreads();
       cta_project<C, NT>(Vr, Vi, n, j + 1, S.wr, S.wi, S.h);
       __syncthreads();
@@ -369,8 +475,9 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       // with 4 outlying values: 44 -> 38) for the same number of restarts
       h.keep = k + (m - k) / 3 < m ? k + (m - k) / 3 : k;
       h.keep_sym = restart_keep(m, k, true);
-      // a symmetric H on the whole CTA, any other on one warp.  Q is written only at the end of hess_core: until then it is the
-      // rotation list and eigenvector scratch (2 m + 2 + m k <= m^2 + 2 m + 2)
+      // a symmetric H on the whole CTA, any other on one warp.  Q is written
+      // only at the end of hess_core: until then it is the rotation list and
+      // eigenvector scratch (2 m + 2 + m k <= m^2 + 2 m + 2)
       const bool sym = sym_eig(h, (double*)S.T, (double*)S.Z, sym_scratch(S.sym, m), tid, NT);
       if (!sym && warp == 0) hess_core(h, S.T, S.Z, S.u, S.key, S.ord, S.Q, lane);
     }
@@ -384,79 +491,93 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       status = OAPB_NOT_CONVERGED;
       break;
     }
-    // V[0..keep] <- V Q[:, 0..keep] in place (each thread owns whole rows r)
+    // V[0..keep] <- V Q[:, 0..keep], f = v_keep beta_hat + f sigma (Sorensen)
     const int keep = S.st->keep;
-    for (int r = tid; r < n; r += NT) {
-      cplx out[kBtMaxM + 1];
-      for (int q = 0; q <= keep; ++q) out[q] = cplx{0, 0};
-      for (int i = 0; i < m; ++i) {
-        const cplx v = {Vr[(long)i * n + r], C ? Vi[(long)i * n + r] : 0.0};
-        for (int q = 0; q <= keep; ++q) out[q] = out[q] + v * S.Q[i + q * m];
+    const cplx bh = S.st->beta_hat, sg = S.st->sigma;
+    for (int r = tid; r < n; r += NT)
+      for (int q0 = 0; q0 <= keep; q0 += kBtCols) {
+        cplx out[kBtCols];
+        cta_combine<C>(Vr, Vi, n, r, m, S.Q, m, q0, keep + 1, out);
+#pragma unroll
+        for (int c = 0; c < kBtCols; ++c) {
+          const int q = q0 + c;
+          if (q < keep) {
+            Nr[(long)q * n + r] = out[c].re;
+            if (C) Ni[(long)q * n + r] = out[c].im;
+          } else if (q == keep) {
+            const cplx nf = out[c] * bh + cplx{S.fr[r], C ? S.fi[r] : 0.0} * sg;
+            S.fr[r] = nf.re;
+            if (C) S.fi[r] = nf.im;
+          }
+        }
       }
-      for (int q = 0; q <= keep; ++q) {
-        Vr[(long)q * n + r] = out[q].re;
-        if (C) Vi[(long)q * n + r] = out[q].im;
-      }
-      // f = v_k beta_hat + f sigma (Sorensen)
-      const cplx f = {S.fr[r], C ? S.fi[r] : 0.0};
-      const cplx nf = out[keep] * S.st->beta_hat + f * S.st->sigma;
-      S.fr[r] = nf.re;
-      if (C) S.fi[r] = nf.im;
-    }
+    double* const tr = Vr;
+    double* const ti = Vi;
+    Vr = Nr;
+    Vi = Ni;
+    Nr = tr;
+    Ni = ti;
     double a2 = 0;
     for (int r = tid; r < n; r += NT) a2 += S.fr[r] * S.fr[r] + (C ? S.fi[r] * S.fi[r] : 0.0);
     fnorm2 = cta_sum2<NT>(a2, 0, S.red).re;
     ++restarts;
     start = keep;
   }
-  // Ritz vectors x_q = V y_q (q < k) in place, then FP64 residuals
+  // Ritz vectors x_q = V y_q (q < k), then FP64 residuals
   double scale = 0;
   for (int q = 0; q < k; ++q) scale = fmax(scale, cabs_(S.ritz[q]));
   if (scale == 0) scale = 1;
   if (status == OAPB_OK || status == OAPB_NOT_CONVERGED) {
-    for (int r = tid; r < n; r += NT) {
-      cplx out[kBtMaxM];
-      for (int q = 0; q < k; ++q) out[q] = cplx{0, 0};
-      for (int i = 0; i < m; ++i) {
-        const cplx v = {Vr[(long)i * n + r], C ? Vi[(long)i * n + r] : 0.0};
-        for (int q = 0; q < k; ++q) out[q] = out[q] + v * S.Y[i + q * m];
+    for (int r = tid; r < n; r += NT)
+      for (int q0 = 0; q0 < k; q0 += kBtCols) {
+        cplx out[kBtCols];
+        cta_combine<C>(Vr, Vi, n, r, m, S.Y, m, q0, k, out);
+#pragma unroll
+        for (int c = 0; c < kBtCols; ++c)
+          if (q0 + c < k) {
+            Nr[(long)(q0 + c) * n + r] = out[c].re;
+            if (C) Ni[(long)(q0 + c) * n + r] = out[c].im;
+          }
       }
-      for (int q = 0; q < k; ++q) {
-        Vr[(long)q * n + r] = out[q].re;
-        if (C) Vi[(long)q * n + r] = out[q].im;
-      }
-    }
-    __syncthreads();
     bool all_ok = true;
-    for (int q = 0; q < k; ++q) {
-      const double* xr = Vr + (long)q * n;
-      const double* xi = Vi + (long)q * n;
-      for (int r = tid; r < n; r += NT) {
-        S.xr[r] = xr[r];
-        if (C) S.xi[r] = xi[r];
-      }
+    for (int q0 = 0; q0 < k; q0 += kBtVerify) {
+      const int nv = k - q0 < kBtVerify ? k - q0 : kBtVerify;
+      double* const br[kBtVerify] = {S.xr, S.wr, S.fr};
+      double* const bi[kBtVerify] = {S.xi, S.wi, S.fi};
       __syncthreads();
-      cta_matvec<C, NT>(P.re, P.im, n, S.xr, S.xi, S.wr, S.wi);
-      ++matvecs;
+      for (int v = 0; v < nv; ++v)
+        for (int r = tid; r < n; r += NT) {
+          const double x = Nr[(long)(q0 + v) * n + r], y = C ? Ni[(long)(q0 + v) * n + r] : 0.0;
+          br[v][r] = x;
+          if (C) bi[v][r] = y;
+          if (P.vre) P.vre[(long)r * k + q0 + v] = x;
+          if (P.vim) P.vim[(long)r * k + q0 + v] = y;
+        }
       __syncthreads();
-      const cplx lam = S.ritz[q];
-      double e2 = 0, x2 = 0;
-      for (int r = tid; r < n; r += NT) {
-        const cplx x = {S.xr[r], C ? S.xi[r] : 0.0};
-        const cplx w = cplx{S.wr[r], C ? S.wi[r] : 0.0} - lam * x;
-        e2 += abs2(w);
-        x2 += abs2(x);
-        if (P.vre) P.vre[(long)r * k + q] = x.re;
-        if (P.vim) P.vim[(long)r * k + q] = x.im;
-      }
-      const cplx sums = cta_sum2<NT>(e2, x2, S.red);
-      const double rr = sqrt(sums.re) / (scale * (sums.im > 0 ? sqrt(sums.im) : 1.0));
-      if (tid == 0) {
-        A.ev_re[(long)P.index * k + q] = lam.re;
-        A.ev_im[(long)P.index * k + q] = lam.im;
-        A.res[(long)P.index * k + q] = rr;
-      }
-      if (!(rr <= A.tol)) all_ok = false;
+      const double* const xr[kBtVerify] = {S.xr, S.wr, S.fr};
+      const double* const xi[kBtVerify] = {S.xi, S.wi, S.fi};
+      cplx lam[kBtVerify], sums[kBtVerify];
+#pragma unroll
+      for (int v = 0; v < kBtVerify; ++v) lam[v] = S.ritz[q0 + (v < nv ? v : 0)];
+      if (nv == 1)
+        cta_residuals<C, NT, 1>(P.re, P.im, n, xr, xi, lam, S.red, sums);
+      else if (nv == 2)
+        cta_residuals<C, NT, 2>(P.re, P.im, n, xr, xi, lam, S.red, sums);
+      else
+        cta_residuals<C, NT, 3>(P.re, P.im, n, xr, xi, lam, S.red, sums);
+      matvecs += nv;
+      ++passes;
+#pragma unroll
+      for (int v = 0; v < kBtVerify; ++v)
+        if (v < nv) {
+          const double rr = sqrt(sums[v].re) / (scale * (sums[v].im > 0 ? sqrt(sums[v].im) : 1.0));
+          if (tid == 0) {
+            A.ev_re[(long)P.index * k + q0 + v] = lam[v].re;
+            A.ev_im[(long)P.index * k + q0 + v] = lam[v].im;
+            A.res[(long)P.index * k + q0 + v] = rr;
+          }
+          if (!(rr <= A.tol)) all_ok = false;
+        }
     }
     if (status == OAPB_OK && !all_ok) status = OAPB_NOT_CONVERGED;
   }
@@ -464,7 +585,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
     A.status[P.index] = status;
     atomicAdd(A.matvecs, matvecs);
     atomicAdd(A.restarts, restarts);
-    atomicAdd(A.op_bytes, matvecs * (unsigned long long)(C ? 16 : 8) * (unsigned long long)n * n);
+    atomicAdd(A.op_bytes, passes * (unsigned long long)(C ? 16 : 8) * (unsigned long long)n * n);
   }
   __syncthreads();
 }
@@ -515,14 +636,14 @@ cudaError_t launch_batched(int v, int grid, size_t smem, cudaStream_t s, const B
   return cudaGetLastError();
 }
 
-// The autotuner's choice per (device, largest n, hdim, wanted, complex):
-// the variant whose launch on a sample of the batch took the least device
+// The autotuner's choice per (device, largest n in steps of 64, hdim, wanted,
+// complex, whether the batch fills the grids): the variant whose launch on a sample of the batch took the least device
 // time (replaces the fixed launch shapes of utils::mapper::SetThreadsBlocks,
 // oapUtils/ThreadsMapper.cpp:36-74).
 struct BatchKey {
-  int dev, nmax, mcap, k, cplx;
+  int dev, nmax, mcap, k, cplx, count;
   bool operator<(const BatchKey& o) const {
-    return std::tie(dev, nmax, mcap, k, cplx) < std::tie(o.dev, o.nmax, o.mcap, o.k, o.cplx);
+    return std::tie(dev, nmax, mcap, k, cplx, count) < std::tie(o.dev, o.nmax, o.mcap, o.k, o.cplx, o.count);
   }
 };
 std::mutex g_bt_mutex;
@@ -541,14 +662,18 @@ void remember_variant(const BatchKey& key, int v) {
   g_bt_choice[key] = v;
 }
 
-// Time every variant on an evenly strided sample of the size-sorted batch
-// (one wave of the default variant's grid) with CUDA events; the sample's
-// outputs land in the batch's output slots and are overwritten by the full
-// launch that follows.  dsample: device room for the sample's descriptors.
+// Time the variants that can win on an evenly strided sample of the
+// size-sorted batch (two waves of the 256 x 2 grid: a sample of one problem per
+// SM hides what more resident CTAs give, and picked 256 x 1, 40.0 ms on 2048
+// problems that 256 x 2 solves in 31.5) with CUDA events; the sample's outputs
+// land in the batch's output slots and are overwritten by the full launch that
+// follows.  256 x 1 (one problem per SM) and 64 x 8 (its registers in local
+// memory) lose at every size tried.  dsample: device room for the sample's
+// descriptors.
 int tune_batched(BatchArgs A, const std::vector<BatchDesc>& d, const int* grids, size_t smem, cudaStream_t s,
                  char* dsample, int* best) {
   const int count = (int)d.size();
-  const int ns = std::min(count, grids[0]);
+  const int ns = std::min(count, 2 * grids[2]);
   std::vector<BatchDesc> sample(ns);
   for (int i = 0; i < ns; ++i) sample[i] = d[(long)i * count / ns];
   if (cudaMemcpyAsync(dsample, sample.data(), sizeof(BatchDesc) * ns, cudaMemcpyHostToDevice, s) != cudaSuccess)
@@ -563,8 +688,9 @@ int tune_batched(BatchArgs A, const std::vector<BatchDesc>& d, const int* grids,
   }
   int rc = OAPB_OK;
   float best_ms = 0;
-  *best = 0;
-  for (int v = 0; v < kBtVariants && !rc; ++v) {
+  *best = 2;
+  for (const int v : {2, 1, 3}) {
+    if (rc) break;
     if (cudaMemsetAsync((void*)A.counter, 0, 4 * sizeof(unsigned long long), s) != cudaSuccess ||
         cudaEventRecord(e0, s) != cudaSuccess ||
         launch_batched(v, std::min(grids[v], ns), smem, s, A) != cudaSuccess ||
@@ -574,7 +700,7 @@ int tune_batched(BatchArgs A, const std::vector<BatchDesc>& d, const int* grids,
     }
     float ms = 0;
     cudaEventElapsedTime(&ms, e0, e1);
-    if (v == 0 || ms < best_ms) {
+    if (v == 2 || ms < best_ms) {
       best_ms = ms;
       *best = v;
     }
@@ -632,16 +758,21 @@ int oapb_arnoldi_solve_batched(const oapb_arnoldi_config* cfg, const oapb_batch_
 
   // one device allocation for descriptors (the batch, then a tuning sample),
   // counters, outputs and the basis slots
-  const size_t vws = sizeof(double) * 2 * (size_t)(mcap + 1) * nmax * gmax;
+  const size_t vws = sizeof(double) * 4 * (size_t)(mcap + 1) * nmax * gmax;
   const size_t nout = (size_t)count * k;
+  // (the outputs lie together: one copy brings them back)
   size_t off_desc = 0, off_cnt = align16(off_desc + sizeof(BatchDesc) * 2 * (size_t)count);
-  size_t off_out = align16(off_cnt + 4 * sizeof(unsigned long long));
-  size_t off_res = align16(off_out + 2 * sizeof(double) * nout);
-  size_t off_st = align16(off_res + sizeof(double) * nout);
+  size_t off_out = off_cnt + 4 * sizeof(unsigned long long);
+  size_t off_res = off_out + 2 * sizeof(double) * nout;
+  size_t off_st = off_res + sizeof(double) * nout;
   size_t off_v = (off_st + sizeof(int) * count + 255) & ~(size_t)255;
   const size_t total = off_v + vws;
   char* buf = nullptr;
-  if (cudaMallocAsync((void**)&buf, total, s) != cudaSuccess) {
+  // (the default pool unmaps the memory at every synchronisation, a millisecond
+  // or more per call)
+  cudaMemPool_t pool = workspace_pool(true);
+  if ((pool ? cudaMallocFromPoolAsync((void**)&buf, total, pool, s) : cudaMallocAsync((void**)&buf, total, s)) !=
+      cudaSuccess) {
     cudaGetLastError();
     return OAPB_ERR_NOMEM;
   }
@@ -677,7 +808,10 @@ int oapb_arnoldi_solve_batched(const oapb_arnoldi_config* cfg, const oapb_batch_
     if (cfg->autotune >= 2) {
       variant = cfg->autotune - 2;
     } else if (cfg->autotune == 1) {
-      const BatchKey key{dev, nmax, mcap, k, any_complex ? 1 : 0};
+      // (sizes of like batches: the largest n to 64, the problems to a power of two)
+      int cl = 0;
+      while ((count >> cl) > 1 && cl < 12) ++cl;
+      const BatchKey key{dev, (nmax + 63) / 64, mcap, k, any_complex ? 1 : 0, cl};
       if (!tuned_variant(key, &variant)) {
         rc = tune_batched(A, d, grids, smem, s, buf + off_desc + sizeof(BatchDesc) * count, &variant);
         if (rc) break;
@@ -691,16 +825,18 @@ int oapb_arnoldi_solve_batched(const oapb_arnoldi_config* cfg, const oapb_batch_
       rc = OAPB_ERR_CUDA;
       break;
     }
-    unsigned long long ctr[4];
-    if (cudaMemcpyAsync(eig_re, A.ev_re, sizeof(double) * nout, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(eig_im, A.ev_im, sizeof(double) * nout, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(residuals, A.res, sizeof(double) * nout, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(status, A.status, sizeof(int) * count, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(ctr, buf + off_cnt, sizeof(ctr), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    std::vector<char> host(off_st + sizeof(int) * count - off_cnt);
+    if (cudaMemcpyAsync(host.data(), buf + off_cnt, host.size(), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess) {
       rc = OAPB_ERR_CUDA;
       break;
     }
+    unsigned long long ctr[4];
+    memcpy(ctr, host.data(), sizeof(ctr));
+    memcpy(eig_re, host.data() + (off_out - off_cnt), sizeof(double) * nout);
+    memcpy(eig_im, host.data() + (off_out - off_cnt) + sizeof(double) * nout, sizeof(double) * nout);
+    memcpy(residuals, host.data() + (off_res - off_cnt), sizeof(double) * nout);
+    memcpy(status, host.data() + (off_st - off_cnt), sizeof(int) * count);
     if (stats) {
       stats->problems = count;
       stats->converged = 0;
