@@ -667,8 +667,8 @@ void remember_variant(const BatchKey& key, int v) {
 // SM hides what more resident CTAs give, and picked 256 x 1, 40.0 ms on 2048
 // problems that 256 x 2 solves in 31.5) with CUDA events; the sample's outputs
 // land in the batch's output slots and are overwritten by the full launch that
-// follows.  256 x 1 (one problem per SM) and 64 x 8 (its registers in local
-// memory) lose at every size tried.  dsample: device room for the sample's
+// follows.  256 x 1 and 64 x 8 (its registers in local memory) lose on every
+// batch of more problems than SMs.  dsample: device room for the sample's
 // descriptors.
 int tune_batched(BatchArgs A, const std::vector<BatchDesc>& d, const int* grids, size_t smem, cudaStream_t s,
                  char* dsample, int* best) {
@@ -807,7 +807,11 @@ int oapb_arnoldi_solve_batched(const oapb_arnoldi_config* cfg, const oapb_batch_
     // launch variant: forced, cached, or timed on a sample of the batch
     if (cfg->autotune >= 2) {
       variant = cfg->autotune - 2;
-    } else if (cfg->autotune == 1) {
+    } else if (cfg->autotune == 1 && (int)count > kNumSMs) {
+      // at most one problem per SM leaves 256 x 1, the default, untimed: there is
+      // no second problem to overlap with and no reason to give up registers
+      // (132 complex problems up to 413 rows: 2.65 ms, 256 x 2 3.25, the others
+      // 4.3 and more).
       // (sizes of like batches: the largest n to 64, the problems to a power of two)
       int cl = 0;
       while ((count >> cl) > 1 && cl < 12) ++cl;
