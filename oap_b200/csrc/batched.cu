@@ -8,7 +8,7 @@
 // decreasing n (largest first, for load balance over uneven sizes) and runs
 // the whole restart loop on the device: Arnoldi steps with CGS + DGKS
 // (rho rule), the restart's small eigenproblem (sym_eig on the whole CTA for a
-// symmetric H, hess_core on one warp for any other), V Q and the residual
+// symmetric H, hess_core on two warps for any other), V Q and the residual
 // update, Ritz vectors and the FP64 residual of every wanted pair.  There are
 // no host round trips between restarts, so no per-restart launch or graph
 // replay exists at all.
@@ -49,6 +49,7 @@ namespace oapb {
 constexpr int kBtVariants = 5;
 constexpr int kBtThreadsOf[kBtVariants] = {256, 128, 256, 128, 64};
 constexpr int kBtMinBlocksOf[kBtVariants] = {1, 2, 2, 4, 8};
+constexpr int kBtHessWarps = 2;  // one more than the rotation chain's: its Z rows
 constexpr int kBtMaxM = 32;
 constexpr int kBtMaxN = 2048;
 
@@ -87,6 +88,7 @@ struct BatchSmem {
   int* order;
   DevState* st;
   void* sym;  // sym_eig scratch
+  SweepShared* ss;
 };
 
 __host__ __device__ __forceinline__ size_t align16(size_t x) { return (x + 15) & ~(size_t)15; }
@@ -105,7 +107,7 @@ __host__ __device__ inline size_t batch_smem_bytes(int nmax, int m) {
   b += 2 * batch_tz_bytes(m);              // T, Z
   b += 4 * (size_t)(m + 1) * sizeof(cplx); // ritz, h, s, u
   b += 2 * (size_t)(m + 1) * sizeof(double) + 64 * sizeof(double);
-  b += 2 * (size_t)(m + 1) * sizeof(int) + sizeof(DevState) + 16 * 17;
+  b += 2 * (size_t)(m + 1) * sizeof(int) + sizeof(DevState) + sizeof(SweepShared) + 16 * 18;
   b += sym_scratch_bytes(m);
   return b;
 }
@@ -140,6 +142,7 @@ __device__ BatchSmem carve(char* base, int nmax, int m) {
   S.order = (int*)take(sizeof(int) * (m + 1));
   S.st = (DevState*)take(sizeof(DevState));
   S.sym = take(sym_scratch_bytes(m));
+  S.ss = (SweepShared*)take(sizeof(SweepShared));
   return S;
 }
 
@@ -352,7 +355,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
   const int n = P.n;
   const int m = n < A.mcap ? n : A.mcap;
   const int k = A.k;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5;
   // two copies of the basis: a restart (and the Ritz vectors) goes from one to
   // the other, so its sums stay in registers a few columns at a time
   const size_t vplane = (size_t)(A.mcap + 1) * A.nmax;
@@ -475,11 +478,12 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       // with 4 outlying values: 44 -> 38) for the same number of restarts
       h.keep = k + (m - k) / 3 < m ? k + (m - k) / 3 : k;
       h.keep_sym = restart_keep(m, k, true);
-      // a symmetric H on the whole CTA, any other on one warp.  Q is written
+      // a symmetric H on the whole CTA, any other on two warps.  Q is written
       // only at the end of hess_core: until then it is the rotation list and
       // eigenvector scratch (2 m + 2 + m k <= m^2 + 2 m + 2)
       const bool sym = sym_eig(h, (double*)S.T, (double*)S.Z, sym_scratch(S.sym, m), tid, NT);
-      if (!sym && warp == 0) hess_core(h, S.T, S.Z, S.u, S.key, S.ord, S.Q, lane);
+      if (!sym && warp < kBtHessWarps)
+        hess_core<cplx, kBtHessWarps>(h, S.T, S.Z, S.u, S.key, S.ord, S.Q, tid, S.ss);
     }
     __syncthreads();
     if (S.st->status & 2) {

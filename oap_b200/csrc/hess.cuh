@@ -27,13 +27,13 @@
 // Work layout: T and Z are column-major with an odd leading dimension
 // hess_ld(m), so a lane-per-column access (row rotations) and a
 // lane-per-row access (column rotations) are both free of bank conflicts.
-// A QR sweep runs its chain of rotations in registers (the 2 x 2 window and
-// the bulge, one shuffle per rotation) while the lanes apply each row
-// rotation to their columns; the column rotations of the sweep, and those on
-// Z, are applied after the chain (each lane the whole sequence to its
-// rows).  The eigenvector back substitutions run one lane per eigenvector
-// (T read by broadcast).  The sweeps run on one warp; for m <= 32 the kernel
-// has four warps, which share the Householder reduction and the product
+// A QR sweep runs its chain of rotations on one warp, in registers (the 2 x 2
+// window and the bulge, one shuffle per rotation) while the lanes apply each
+// row rotation to their columns; the column rotations of the sweep, and those
+// on Z, are applied after the chain (each lane the whole sequence to its row),
+// those on Z by another warp beside the next sweep.  The eigenvector back
+// substitutions run one lane per eigenvector (T read by broadcast).  For m <= 32
+// the kernel's four warps share the Householder reduction and the product
 // Y = Z U.
 //
 // Every loop is bounded (30 m sweeps for the Schur form); hitting the bound
@@ -69,8 +69,8 @@ struct HessArgs {
 // wanted.  It takes most of what more would give (over 32 operators with 8 of
 // 24 at a spectrum's edge, 7800 applications with none, 5600 with one, 4600
 // with five; more of them also leave a warm start little to save).  On the
-// general path a restart costs as much as 20 - 40 applications (its one-warp
-// Schur form), and more kept vectors mean more restarts: the wanted alone.
+// general path a restart costs as much as 10 - 30 applications (its Schur
+// form), and more kept vectors mean more restarts: the wanted alone.
 __host__ __device__ inline int restart_keep(int m, int k, bool sym) { return sym && k + 1 < m ? k + 1 : k; }
 
 // leading dimension of the T / Z work arrays (odd)
@@ -116,21 +116,24 @@ __device__ __forceinline__ Cx cfma2(Cx a, Cx b, Cx c, Cx d) {
   return cfma(a, b, c * d);
 }
 
-// The rotation of givens() (p x + q y = sqrt(|x|^2 + |y|^2), p = conj(x) / r,
-// q = conj(y) / r) for entries of a matrix that hess_core has scaled to a
-// largest entry in [1, 2): the sum of squares cannot overflow, and a pair
-// whose squares sum below tiny2 (far below the working precision relative
-// to the matrix) gives the identity.  No branch: the sweep's rotation chain
-// stays one straight block of instructions.
-template <typename Cx>
-__device__ __forceinline__ void givens_s(Cx x, Cx y, Cx& p, Cx& q) {
-  using R = decltype(Cx::re);
-  const R r2 = fma_t(x.re, x.re, fma_t(x.im, x.im, fma_t(y.re, y.re, y.im * y.im)));
-  const bool ok = r2 > HessK<R>::tiny2;
-  const R ir = rsqrt_t(ok ? r2 : R(1));
-  p = ok ? Cx{x.re * ir, -x.im * ir} : Cx{1, 0};
-  q = ok ? Cx{y.re * ir, -y.im * ir} : Cx{0, 0};
+// p, known to lie in shared memory: its accesses then need no generic address
+template <typename P>
+__device__ __forceinline__ P* as_shared(P* p) {
+  return static_cast<P*>(__cvta_shared_to_generic(__cvta_generic_to_shared(p)));
 }
+
+// one complex entry in one access (T, Z and the rotation lists start on 16
+// bytes; the structs alone promise only a component's alignment)
+__device__ __forceinline__ cplx cload(const cplx* p) {
+  const double2 v = *reinterpret_cast<const double2*>(p);
+  return {v.x, v.y};
+}
+__device__ __forceinline__ cplxf cload(const cplxf* p) {
+  const float2 v = *reinterpret_cast<const float2*>(p);
+  return {v.x, v.y};
+}
+__device__ __forceinline__ void cstore(cplx* p, cplx v) { *reinterpret_cast<double2*>(p) = make_double2(v.re, v.im); }
+__device__ __forceinline__ void cstore(cplxf* p, cplxf v) { *reinterpret_cast<float2*>(p) = make_float2(v.re, v.im); }
 
 // principal square root of z (prescaled entries: |z| stays far inside the
 // range), re >= 0
@@ -194,138 +197,218 @@ static __device__ int find_split(const Cx* T, int ld, int h, int lane) {
 
 // One single-shift QR sweep on the active window [l, h] of Hessenberg T,
 // applied to whole rows / columns of T (the final T is G T G^H with G =
-// G_{h-1} ... G_l); Z <- Z G_l^H ... G_{h-1}^H.  rot: 2 m cplx of scratch.
-// T must be prescaled (hess_core): the rotations come from givens_s.
+// G_{h-1} ... G_l); Z <- Z G_l^H ... G_{h-1}^H.
+// T must be prescaled (hess_core).
 //
-// The rotations form a dependent chain: rotation k needs the bulge pair
-// left by rotation k - 1.  That chain runs in registers: every lane carries
-// the 2 x 2 window T[k..k+1][k..k+1] and the bulge through the algebra of
-// one rotation on both sides, and the one entry of the window that earlier
-// rotations reach from outside it, T[k][k+1], comes from the lane that owns
-// column k + 1.  The matrix itself is updated off the chain: while the chain
-// runs, lane c applies each row rotation to column c (its row-k entry carried
-// in a register, the row-(k+1) entry read once), and after the chain one
-// lane per row applies all column rotations to its row of T and of Z.  Left
-// and right rotations commute, so the result is G T G^H as in the
-// interleaved sweep; the entries below the subdiagonal that the interleaved
-// sweep never fills come out of this order at rounding level and are set
-// to zero.  The loop over rotations l .. h-2 has no branch (the last
-// rotation, which has no next window, is peeled): a single warp issues it
-// as one straight block, so the row updates fill the chain's latency.
-// NT: columns per lane (c = lane + 32 t, t < NT); m <= 32 NT.  WZ: Z is
-// updated (Z non-null).
-template <typename Cx, int NT, bool WZ>
-static __device__ __forceinline__ void warp_sweep_nt(Cx* T, Cx* Z, int m, int ld, int l, int h, Cx mu, Cx* rot,
-                                                     int lane) {
+// warp_chain: the rotations (p, q at rot[2 k], rot[2 k + 1]) and their left
+// products.  Rotation k needs the bulge pair left by rotation k - 1, so they
+// form a dependent chain, which bounds the sweep.  It runs in registers:
+// every lane carries the pair (x, y) = (T[k][k-1], T[k+1][k-1]) and the
+// window D = T[k][k], F = T[k+1][k], G = T[k+1][k+1] (E = T[k][k+1] comes from
+// the lane that owns column k + 1).  With r^2 = |x|^2 + |y|^2 and the
+// unnormalised row N1 = x F - y D, N2 = x G - y E, the next pair's x is
+// (N1 x + N2 y) / r^2 and the next D is (N2 conj(x) - N1 conj(y)) / r^2: both
+// need only products that run beside the reciprocal square root, one
+// multiplication after it.  A pair whose squares sum below tiny2 (far below
+// the working precision relative to the matrix) gives the identity.
+// Meanwhile lane c applies each row rotation to column c (its row-k entry
+// carried in a register); rows k + 2 and on are read a step ahead.
+//
+// cols_rows: after the chain, one lane per row applies all column rotations to
+// its row of T or Z.  Left and right rotations commute, so the result is
+// G T G^H as in the interleaved sweep; the entries below the subdiagonal that
+// the interleaved sweep never fills come out of this order at rounding level
+// and are set to zero.  With several warps only the chain is serial: the next
+// sweep starts when the rows of T are done, and the rows of Z go to another
+// warp, which works beside it (two rotation lists in turn).
+//
+// Clocks per rotation at m = 32, FP64 (FP32): one warp, the window normalised
+// before its products and the column rotations of T and Z after the chain, 457
+// + 265 (323 + 211); now 334 + 112 (197 + 72), at m = 64 413 + 104 before 582 +
+// 487.  A Schur form with 24 exact shifts, m = 32: 1114 -> 720 us (714 -> 395);
+// m = 64, 56 shifts: 6.13 -> 3.06 ms (3.93 -> 1.58).  An FP64 instruction holds
+// a warp's FP64 port for about 4 clocks: the chain's 80 are what bounds it.
+// (Column rotations of T inside the chain's loop, a step behind it, made that
+// 512 clocks per rotation.)
+// NT: columns per lane (c = lane + 32 t, t < NT); m <= 32 NT.
+template <typename Cx, int NT>
+static __device__ __forceinline__ void warp_chain(Cx* T, int m, int ld, int l, int h, Cx mu, Cx* rot, int lane) {
+  using R = decltype(Cx::re);
   const int nt = (m + 31) >> 5;
   const Cx zero = {0, 0};
-  Cx carry[NT], b[NT];
+  Cx carry[NT], b[NT], bn[NT];
   bool own[NT];
+  const int r2nd = l + 2 < h ? l + 2 : h;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
     const int c = lane + 32 * t;
     own[t] = t < nt && c >= l && c < m;
-    carry[t] = own[t] ? TT_(l, c) : zero;
-    b[t] = own[t] ? TT_(l + 1, c) : zero;
+    carry[t] = own[t] ? cload(&TT_(l, c)) : zero;
+    b[t] = own[t] ? cload(&TT_(l + 1, c)) : zero;
+    bn[t] = own[t] ? cload(&TT_(r2nd, c)) : zero;
   }
-  Cx D = TT_(l, l), E = TT_(l, l + 1), F = TT_(l + 1, l), G = TT_(l + 1, l + 1);
+  Cx D = cload(&TT_(l, l)), F = cload(&TT_(l + 1, l)), G = cload(&TT_(l + 1, l + 1));
+  Cx s2 = cload(&TT_(r2nd, l + 1)), g2 = cload(&TT_(r2nd, r2nd));
   Cx x = D - mu, y = F;
-  int k = l;
-  for (; k + 1 < h; ++k) {
-    // inputs of this step from rows k + 1, k + 2 (not written before it)
-    Cx bn[NT];
+  for (int k = l;; ++k) {
+    // the step after the next one's inputs: row k + 3 (the last row instead
+    // beyond the window, not used then)
+    const int rn = k + 3 < h ? k + 3 : h, cn = rn - 1;
+    Cx bnn[NT];
 #pragma unroll
-    for (int t = 0; t < NT; ++t) bn[t] = own[t] ? TT_(k + 2, lane + 32 * t) : zero;
-    const Cx s2 = TT_(k + 2, k + 1), g2 = TT_(k + 2, k + 2), t2 = TT_(k + 1, k + 2);
-    // row k's entry of column k + 2 before this rotation
-    const int c2 = k + 2;
+    for (int t = 0; t < NT; ++t) bnn[t] = own[t] ? cload(&TT_(rn, lane + 32 * t)) : zero;
+    const Cx s3 = cload(&TT_(rn, cn)), g3 = cload(&TT_(rn, rn));
+    // row k's entry of column k + 1
+    const int c1 = k + 1;
     Cx e = carry[0];
 #pragma unroll
     for (int t = 1; t < NT; ++t)
-      if (t == (c2 >> 5)) e = carry[t];
-    const Cx epre = shfl_c(e, c2 & 31);
-    Cx p, q;
-    givens_s(x, y, p, q);
-    rot[2 * k] = p;  // every lane stores the same values
-    rot[2 * k + 1] = q;
-    const Cx pc = conj(p), qc = conj(q), nqc = -qc;
-    // the window through rotation k on both sides, then the next one
-    const Cx F1 = cfma2(nqc, D, pc, F), G1 = cfma2(nqc, E, pc, G);
-    x = cfma2(F1, pc, G1, qc);   // T[k+1][k]
-    y = s2 * qc;                 // T[k+2][k], the bulge
-    D = cfma2(-F1, q, G1, p);    // T[k+1][k+1]
-    F = s2 * p;                  // T[k+2][k+1]
-    G = g2;                      // T[k+2][k+2]
-    E = cfma2(nqc, epre, pc, t2);  // T[k+1][k+2] after row rotation k
+      if (t == (c1 >> 5)) e = carry[t];
+    const Cx E = shfl_c(e, c1 & 31);
+    const R r2 = fma_t(x.re, x.re, x.im * x.im) + fma_t(y.re, y.re, y.im * y.im);
+    const Cx ny = -y;
+    const Cx N1 = cfma2(ny, D, x, F), N2 = cfma2(ny, E, x, G);
+    const Cx X = cfma2(N1, x, N2, y), Dn = cfma2(N2, conj(x), -N1, conj(y));
+    const bool ok = r2 > HessK<R>::tiny2;
+    const R ir = rsqrt_t(ok ? r2 : R(1));
+    const R ir2 = ir * ir;
+    const Cx p = ok ? Cx{x.re * ir, -x.im * ir} : Cx{1, 0};
+    const Cx q = ok ? Cx{y.re * ir, -y.im * ir} : zero;
+    cstore(rot + 2 * k, p);  // every lane stores the same values
+    cstore(rot + 2 * k + 1, q);
+    x = ok ? ir2 * X : F;
+    D = ok ? ir2 * Dn : G;
+    y = s2 * conj(q);  // T[k+2][k], the bulge
+    F = s2 * p;        // T[k+2][k+1]
+    G = g2;
+    s2 = s3;
+    g2 = g3;
+    const Cx pc = conj(p), nqc = -conj(q);
     // row rotation k on the lanes' columns (rows k, k + 1)
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      if (own[t]) {
-        TT_(k, lane + 32 * t) = cfma2(p, carry[t], q, b[t]);
-        carry[t] = cfma2(nqc, carry[t], pc, b[t]);
-      }
+      const Cx top = cfma2(p, carry[t], q, b[t]);
+      carry[t] = cfma2(nqc, carry[t], pc, b[t]);
+      if (own[t]) cstore(&TT_(k, lane + 32 * t), top);
       b[t] = bn[t];
+      bn[t] = bnn[t];
     }
+    if (k + 1 >= h) break;
   }
-  {  // rotation h - 1
-    Cx p, q;
-    givens_s(x, y, p, q);
-    rot[2 * k] = p;
-    rot[2 * k + 1] = q;
-    const Cx pc = conj(p), nqc = -conj(q);
 #pragma unroll
-    for (int t = 0; t < NT; ++t) {
-      if (own[t]) {
-        TT_(k, lane + 32 * t) = cfma2(p, carry[t], q, b[t]);
-        TT_(h, lane + 32 * t) = cfma2(nqc, carry[t], pc, b[t]);
-      }
-    }
+  for (int t = 0; t < NT; ++t)
+    if (own[t]) cstore(&TT_(h, lane + 32 * t), carry[t]);
+}
+
+// U column rotations from k0 on, on one row (t: its entry of column 0; c: its
+// entry of column k0, then of k0 + U); all are read before the first is stored
+template <typename Cx, bool WT, int U>
+static __device__ __forceinline__ void cols_block(Cx* t, int ld, int i, int k0, const Cx* rot, Cx& c) {
+  const Cx zero = {0, 0};
+  Cx p[U], q[U], nb[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    p[u] = cload(rot + 2 * (k0 + u));
+    q[u] = cload(rot + 2 * (k0 + u) + 1);
+    nb[u] = cload(t + (k0 + u + 1) * ld);
   }
-  __syncwarp();
-  // column rotations l .. h-1 on rows 0 .. h of T and on every row of Z (one
-  // lane per row); the entries below the subdiagonal of the window (rows
-  // i >= k + 2 of column k) are set to zero.  Rows below h hold zeros in
-  // these columns: their T stores are skipped.
-  for (int i = lane; i < m; i += 32) {
-    const bool trow = i <= h;
-    Cx c = TT_(i, l);
-    Cx cz = WZ ? ZZ_(i, l) : zero;
-    for (int kk = l; kk < h; ++kk) {
-      const Cx p = rot[2 * kk], q = rot[2 * kk + 1], pc = conj(p), qc = conj(q);
-      const Cx nb = TT_(i, kk + 1);
-      const Cx tk = cfma2(c, pc, nb, qc);
-      if (trow) TT_(i, kk) = kk + 2 <= i ? zero : tk;
-      c = cfma2(-c, q, nb, p);
-      if (WZ) {
-        const Cx z1 = ZZ_(i, kk + 1);
-        ZZ_(i, kk) = cfma2(cz, pc, z1, qc);
-        cz = cfma2(-cz, q, z1, p);
-      }
-    }
-    if (trow) TT_(i, h) = c;
-    if (WZ) ZZ_(i, h) = cz;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const Cx v = cfma2(c, conj(p[u]), nb[u], conj(q[u]));
+    cstore(t + (k0 + u) * ld, WT && k0 + u + 2 <= i ? zero : v);
+    c = cfma2(-c, q[u], nb[u], p[u]);
   }
+}
+
+// column rotations l .. h-1 on row i of T (WT, i <= h; the entries below the
+// window's subdiagonal, rows i >= k + 2 of column k, are set to zero, and rows
+// below h hold zeros in these columns) or of Z
+template <typename Cx, bool WT>
+static __device__ __forceinline__ void cols_rows(Cx* M, int ld, int i, int l, int h, const Cx* rot) {
+  Cx* t = M + i;
+  Cx c = cload(t + l * ld);
+  int k = l;
+  for (; k + 4 <= h; k += 4) cols_block<Cx, WT, 4>(t, ld, i, k, rot, c);
+  if (k + 2 <= h) {
+    cols_block<Cx, WT, 2>(t, ld, i, k, rot, c);
+    k += 2;
+  }
+  if (k < h) cols_block<Cx, WT, 1>(t, ld, i, k, rot, c);
+  cstore(t + h * ld, c);
+}
+
+// barriers of the NW warps of a multi-warp small eigensolver (named barriers 1
+// and, between the sweeps, 2: the rest of a block may use barrier 0)
+__device__ __forceinline__ void hess_bar(int nthr) { asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory"); }
+__device__ __forceinline__ void sweep_bar(int nthr) { asm volatile("bar.sync 2, %0;" ::"r"(nthr) : "memory"); }
+
+// what the leading warp of a multi-warp hess_core tells the others
+constexpr int kHessWarps = 4;
+struct SweepShared {
+  int l[2], h[2];  // the window of each rotation list's sweep; l < 0: no more sweeps
+  int ok, sym;
+  double scale;
+  double mx[kHessWarps];
+};
+// the sweeps' state: two rotation lists used in turn
+template <typename Cx>
+struct Sweeps {
+  Cx* rot[2];
+  SweepShared* ss;
+  int buf;
+};
+
+// The column rotations of one sweep on NW warps: 32 rows of T per warp, then
+// (the next sweep may start) 32 rows of Z per warp, the leading warp last.
+template <typename Cx, int NW>
+static __device__ __forceinline__ void sweep_cols(Cx* T, Cx* Z, int m, int ld, int l, int h, const Cx* rot, int warp,
+                                                  int lane) {
+  for (int i = 32 * warp + lane; i <= h; i += 32 * NW) cols_rows<Cx, true>(T, ld, i, l, h, rot);
+  if (m > 32) sweep_bar(32 * NW);
+  for (int i = 32 * (NW - 1 - warp) + lane; i < m; i += 32 * NW) cols_rows<Cx, false>(Z, ld, i, l, h, rot);
   __syncwarp();
 }
 
-// the carries stay in registers when their count is fixed by m's range
-template <typename Cx, bool WZ>
-static __device__ void warp_sweep_z(Cx* T, Cx* Z, int m, int ld, int l, int h, Cx mu, Cx* rot, int lane) {
+template <typename Cx, int NW>
+static __device__ __forceinline__ void warp_sweep(Cx* T, Cx* Z, int m, int ld, int l, int h, Cx mu, Sweeps<Cx>& sw,
+                                                  int lane) {
+  Cx* rot = sw.rot[sw.buf];
+  // (the carries stay in registers when their count is fixed by m's range)
   if (m <= 32)
-    warp_sweep_nt<Cx, 1, WZ>(T, Z, m, ld, l, h, mu, rot, lane);
+    warp_chain<Cx, 1>(T, m, ld, l, h, mu, rot, lane);
   else if (m <= 64)
-    warp_sweep_nt<Cx, 2, WZ>(T, Z, m, ld, l, h, mu, rot, lane);
+    warp_chain<Cx, 2>(T, m, ld, l, h, mu, rot, lane);
   else if (m <= 128)
-    warp_sweep_nt<Cx, 4, WZ>(T, Z, m, ld, l, h, mu, rot, lane);
+    warp_chain<Cx, 4>(T, m, ld, l, h, mu, rot, lane);
   else
-    warp_sweep_nt<Cx, kMaxM / 32, WZ>(T, Z, m, ld, l, h, mu, rot, lane);
+    warp_chain<Cx, kMaxM / 32>(T, m, ld, l, h, mu, rot, lane);
+  __syncwarp();
+  if (lane == 0) {
+    sw.ss->l[sw.buf] = l;
+    sw.ss->h[sw.buf] = h;
+  }
+  sweep_bar(32 * NW);
+  sweep_cols<Cx, NW>(T, Z, m, ld, l, h, rot, 0, lane);
+  sw.buf ^= 1;
 }
-template <typename Cx>
-static __device__ void warp_sweep(Cx* T, Cx* Z, int m, int ld, int l, int h, Cx mu, Cx* rot, int lane) {
-  if (Z)
-    warp_sweep_z<Cx, true>(T, Z, m, ld, l, h, mu, rot, lane);
-  else
-    warp_sweep_z<Cx, false>(T, Z, m, ld, l, h, mu, rot, lane);
+
+// the other warps' side of the leading warp's sweeps, until it ends them
+template <typename Cx, int NW>
+static __device__ __forceinline__ void help_sweeps(Cx* T, Cx* Z, int m, int ld, Sweeps<Cx>& sw, int warp, int lane) {
+  for (;;) {
+    sweep_bar(32 * NW);
+    const int l = sw.ss->l[sw.buf], h = sw.ss->h[sw.buf];
+    const Cx* rot = sw.rot[sw.buf];
+    sw.buf ^= 1;
+    if (l < 0) return;
+    sweep_cols<Cx, NW>(T, Z, m, ld, l, h, rot, warp, lane);
+  }
+}
+template <typename Cx, int NW>
+static __device__ void end_sweeps(Sweeps<Cx>& sw, int lane) {
+  if (lane == 0) sw.ss->l[sw.buf] = -1;
+  sweep_bar(32 * NW);
+  sw.buf ^= 1;
 }
 
 // Householder reduction of dense T to Hessenberg form, Z accumulating.
@@ -387,10 +470,6 @@ static __device__ void warp_hessenberg(Cx* T, Cx* Z, Cx* v, int m, int ld, int l
     __syncwarp();
   }
 }
-
-// barrier of the NW warps of a multi-warp small eigensolver (named barrier
-// 1: the rest of a block may use barrier 0)
-__device__ __forceinline__ void hess_bar(int nthr) { asm volatile("bar.sync 1, %0;" ::"r"(nthr) : "memory"); }
 
 // The Householder reduction on NW warps (m <= 32, all NW warps calling;
 // warp 0 forms each reflector): per step, P T has one lane per column and
@@ -485,8 +564,8 @@ static __device__ void block_hessenberg32(Cx* T, Cx* Z, Cx* v, Cx* part, decltyp
 }
 
 // Complex Schur form in place; returns false when the sweep budget ran out.
-template <typename Cx>
-static __device__ bool warp_schur(Cx* T, Cx* Z, int m, int ld, Cx* rot, int lane) {
+template <typename Cx, int NW>
+static __device__ __forceinline__ bool warp_schur(Cx* T, Cx* Z, int m, int ld, Sweeps<Cx>& sw, int lane) {
   using R = decltype(Cx::re);
   int h = m - 1, its = 0, total = 0;
   while (h > 0) {
@@ -508,7 +587,7 @@ static __device__ bool warp_schur(Cx* T, Cx* Z, int m, int ld, Cx* rot, int lane
     const Cx m1 = tr2 + disc, m2 = tr2 - disc;
     Cx mu = abs2(m1 - d) < abs2(m2 - d) ? m1 : m2;
     if (its > 0 && its % 10 == 0) mu = d + Cx{sqrt_t(abs2(c)), 0};
-    warp_sweep(T, Z, m, ld, l, h, mu, rot, lane);
+    warp_sweep<Cx, NW>(T, Z, m, ld, l, h, mu, sw, lane);
     ++its;
   }
   __syncwarp();
@@ -806,29 +885,32 @@ static __device__ double warp_zu(const Cx* Z, int m, int ld, const Cx* U, int W,
   return maxest;
 }
 
-// Shared scratch of the multi-warp (NW > 1) hess_core beyond its workspaces.
+// Shared scratch of block_hessenberg32.
 template <typename Cx, int NW>
-struct HessShared {
+struct HouseShared {
   Cx v[32];
   Cx part[2 * NW * 32];
   decltype(Cx::re) f;
-  double mx[NW];
-  double scale;
-  int ok;
 };
 
-// The body of k_hess on NW warps (tid = 0 .. 32 NW - 1 of the calling
+// The body of k_hess on NW >= 2 warps (tid = 0 .. 32 NW - 1 of the calling
 // threads), with its workspaces passed in: T, Z (leading dimension
 // hess_ld(m), m columns each), u (m), key (m), ord (m), scratch
-// (hess_scratch_cplx(m)); hs (NW > 1 only): shared scratch.  Callable from
-// any kernel by one full warp (NW = 1) or by NW full warps when m <= 32; the
-// outputs in `a` may point to shared or global memory.  With NW > 1 the
-// Householder reduction and the product Y = Z U run on all warps, the Schur
-// sweeps, the sort and the back substitutions on warp 0; the other warps
-// return before the exact shifts.
-template <typename Cx, int NW = 1>
+// (hess_scratch_cplx(m); 2 m + 2 + m max(2, min(nvec, 32)) of it are used).
+// SH: T, Z and the scratch lie in shared memory.
+// Callable from any kernel by NW full warps, with shared scratch ss and, for
+// a dense input of m <= 32, hs; the outputs in `a` may point to shared or
+// global memory.  The sweeps' column rotations and, for m <= 32, the
+// Householder reduction and the product Y = Z U run on all warps; the rotation
+// chains, the sort and the back substitutions on warp 0.
+template <typename Cx, int NW, bool SH = true>
 static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double* key, int* ord, Cx* scratch,
-                                 int tid, HessShared<Cx, NW>* hs = nullptr) {
+                                 int tid, SweepShared* ss, HouseShared<Cx, NW>* hs = nullptr) {
+  if constexpr (SH) {
+    T = as_shared(T);
+    Z = as_shared(Z);
+    scratch = as_shared(scratch);
+  }
   using R = decltype(Cx::re);
   constexpr int nthr = NW * 32;
   const int lane = tid & 31, warp = tid >> 5;
@@ -836,7 +918,8 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
   const long mm = (long)m * m;
   DevState* st = a.st;
   Cx* rot = scratch;           // 2 m
-  Cx* U = scratch + 2 * m + 2; // m x 32
+  Cx* U = scratch + 2 * m + 2; // m x 32; the second rotation list during the sweeps
+  Sweeps<Cx> sw{{rot, U}, ss, 0};
 
   // T = sig H with sig a power of two that puts the largest |re| or |im| of
   // H in [1, 2): exact, and the Schur sweeps' rotations and shifts then need
@@ -855,12 +938,12 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
     TT_(r, c) = cx_from<Cx>(sig * a.Hin[i]);
     ZZ_(r, c) = (r == c) ? Cx{1, 0} : Cx{0, 0};
   }
-  if constexpr (NW > 1) {
+  hess_bar(nthr);
+  if (a.dense && m <= 32 && hs) {
+    block_hessenberg32<Cx, NW>(T, Z, hs->v, hs->part, &hs->f, m, ld, warp, lane);
+  } else if (a.dense) {
+    if (warp == 0) warp_hessenberg(T, Z, u, m, ld, lane);
     hess_bar(nthr);
-    if (a.dense) block_hessenberg32<Cx, NW>(T, Z, hs->v, hs->part, &hs->f, m, ld, warp, lane);
-  } else {
-    __syncwarp();
-    if (a.dense) warp_hessenberg(T, Z, u, m, ld, lane);
   }
   const int nvec = a.nvec > k ? (a.nvec < m ? a.nvec : m) : k;
   const int W = nvec < 32 ? nvec : 32;
@@ -875,6 +958,8 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
   if (warp == 0) {
     sym = !a.dense && a.tol > 0 && warp_is_hermitian(T, m, ld, 0.1 * a.tol, lane);
     if (sym && lane == 0) st->symtri += 1;
+    if (lane == 0) ss->sym = sym;
+    sweep_bar(nthr);
     bool ok;
     if (sym) {
       symtri_load(T, Z, m, ld, sd, se, lane);
@@ -884,15 +969,14 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
         symtri_store(T, m, ld, sd, se, lane);
       }
     } else {
-      ok = warp_schur(T, Z, m, ld, rot, lane);
+      ok = warp_schur<Cx, NW>(T, Z, m, ld, sw, lane);
+      end_sweeps<Cx, NW>(sw, lane);
     }
     if (!ok && lane == 0) {
       st->status |= 2;
       st->converged = 0;
     }
-    if constexpr (NW > 1) {
-      if (lane == 0) hs->ok = ok;
-    }
+    if (lane == 0) ss->ok = ok;
     if (ok) {
       // sort order of diag(T)
       for (int i = lane; i < m; i += 32) {
@@ -920,26 +1004,23 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
       for (int o = 16; o > 0; o >>= 1) tnorm = fmax(tnorm, __shfl_xor_sync(0xffffffffu, tnorm, o));
       small = (double)HessK<R>::eps * (tnorm > 0 ? tnorm : 1.0);
       warp_backsub(T, m, ld, ord, nvec, 0, small, U, lane);
-      if constexpr (NW > 1) {
-        if (lane == 0) hs->scale = scale;
-      }
+      if (lane == 0) ss->scale = scale;
     }
     __syncwarp();
+  } else {
+    sweep_bar(nthr);
+    sym = ss->sym;
+    if (!sym) help_sweeps<Cx, NW>(T, Z, m, ld, sw, warp, lane);
   }
   double maxest = 0;
-  if constexpr (NW > 1) {
-    // eigenvectors of the first nvec Ritz values (the wanted k and optional
-    // guard vectors; nvec <= m <= 32) on all warps
-    hess_bar(nthr);
-    if (!hs->ok) return;
-    scale = hs->scale;
-    const double me = warp_zu(Z, m, ld, U, W, 0, nvec, k, beta, scale, a.Y, a.est, warp, NW, lane);
-    if (lane == 0) hs->mx[warp] = me;
-    hess_bar(nthr);
-    if (warp != 0) return;
-    for (int w = 0; w < NW; ++w) maxest = fmax(maxest, hs->mx[w]);
-  } else {
-    if (scale == 0) return;  // the Schur sweeps ran out (status set)
+  hess_bar(nthr);
+  if (!ss->ok) return;  // the Schur sweeps ran out (status set)
+  scale = ss->scale;
+  // eigenvectors of the first nvec Ritz values (the wanted k and optional
+  // guard vectors), for m <= 32 on all warps
+  if (m <= 32) {
+    maxest = warp_zu(Z, m, ld, U, W, 0, nvec, k, beta, scale, a.Y, a.est, warp, NW, lane);
+  } else if (warp == 0) {
     for (int q0 = 0; q0 < nvec; q0 += 32) {
       if (q0 > 0) {
         warp_backsub(T, m, ld, ord, nvec, q0, small, U, lane);
@@ -950,8 +1031,11 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
       __syncwarp();
     }
   }
+  if (lane == 0) ss->mx[warp] = maxest;
+  hess_bar(nthr);
+  for (int w = 0; w < NW; ++w) maxest = fmax(maxest, ss->mx[w]);
   const int conv = maxest <= a.tol;
-  if (lane == 0) {
+  if (tid == 0) {
     st->converged = conv;
     st->scale = scale;
     st->maxest = maxest;
@@ -960,15 +1044,23 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
 
   // exact shifts on H with the unwanted Ritz values (kept in u[] before T
   // is reloaded with H)
-  __syncwarp();
-  for (int q = lane; q < m; q += 32) u[q] = TT_(ord[q], ord[q]);
-  __syncwarp();
-  for (long i = lane; i < mm; i += 32) {
+  if (warp == 0) {
+    __syncwarp();
+    for (int q = lane; q < m; q += 32) u[q] = TT_(ord[q], ord[q]);
+    __syncwarp();
+  }
+  hess_bar(nthr);
+  for (long i = tid; i < mm; i += nthr) {
     const int r = (int)(i % m), c = (int)(i / m);
     TT_(r, c) = cx_from<Cx>(sig * a.Hin[i]);
     ZZ_(r, c) = (r == c) ? Cx{1, 0} : Cx{0, 0};
   }
-  __syncwarp();
+  hess_bar(nthr);
+  if (warp != 0) {
+    if (!sym) help_sweeps<Cx, NW>(T, Z, m, ld, sw, warp, lane);
+    hess_bar(nthr);
+    return;
+  }
   if (sym) {  // the same exact shifts as implicit symmetric tridiagonal steps
     symtri_load(T, Z, m, ld, sd, se, lane);
     for (int q = a.keep; q < m; ++q) {
@@ -998,12 +1090,13 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
         const int l = find_split(T, ld, hb, lane);
         if (l > 0 && lane == 0) TT_(l, l - 1) = Cx{0, 0};
         __syncwarp();
-        if (l < hb) warp_sweep(T, Z, m, ld, l, hb, mu, rot, lane);
+        if (l < hb) warp_sweep<Cx, NW>(T, Z, m, ld, l, hb, mu, sw, lane);
         hb = l - 1;
       }
     }
+    end_sweeps<Cx, NW>(sw, lane);
   }
-  __syncwarp();
+  hess_bar(nthr);  // the other warps' rows of Z are in place
   if (lane == 0) {
     st->beta_hat = isig * cx_to(TT_(a.keep, a.keep - 1));
     st->sigma = cx_to(ZZ_(m - 1, a.keep - 1));
@@ -1017,9 +1110,8 @@ static __device__ void hess_core(const HessArgs& a, Cx* T, Cx* Z, Cx* u, double*
   }
 }
 
-// warps of k_hess / k_hess_f32 for m <= 32 (one warp above)
-constexpr int kHessWarps = 4;
-__host__ __device__ inline int hess_threads(int m) { return m <= 32 ? 32 * kHessWarps : 32; }
+// threads of k_hess / k_hess_f32
+__host__ __device__ inline int hess_threads(int) { return 32 * kHessWarps; }
 
 // dynamic shared memory (or a.gws): T, Z, scratch of the working type Cx;
 // launched with hess_threads(m) threads
@@ -1028,13 +1120,13 @@ static __device__ void hess_kernel_body(const HessArgs& a, unsigned char* dyn) {
   __shared__ Cx u[kMaxM];
   __shared__ double key[kMaxM];
   __shared__ int ord[kMaxM];
-  __shared__ HessShared<Cx, kHessWarps> hs;
-  Cx* T = a.gws ? reinterpret_cast<Cx*>(a.gws) : reinterpret_cast<Cx*>(dyn);
+  __shared__ SweepShared ss;
+  __shared__ HouseShared<Cx, kHessWarps> hs;
   const size_t tz = (size_t)hess_ld(a.m) * a.m;
-  if (blockDim.x == 32 * kHessWarps && a.m <= 32)
-    hess_core<Cx, kHessWarps>(a, T, T + tz, u, key, ord, T + 2 * tz, threadIdx.x, &hs);
-  else if (threadIdx.x < 32)
-    hess_core<Cx, 1>(a, T, T + tz, u, key, ord, T + 2 * tz, threadIdx.x);
+  if (Cx* T = reinterpret_cast<Cx*>(a.gws))
+    hess_core<Cx, kHessWarps, false>(a, T, T + tz, u, key, ord, T + 2 * tz, threadIdx.x, &ss, &hs);
+  else if (Cx* S = reinterpret_cast<Cx*>(dyn))
+    hess_core<Cx, kHessWarps>(a, S, S + tz, u, key, ord, S + 2 * tz, threadIdx.x, &ss, &hs);
 }
 
 // FP64 working arithmetic (the restart loop and the refinement)

@@ -1918,7 +1918,8 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
       rc |= OAPB_ERR_CUDA;
   }
   const size_t static_smem =
-      kMaxM * (sizeof(cplx) + sizeof(double) + sizeof(int)) + sizeof(HessShared<cplx, kHessWarps>) + 1024;
+      kMaxM * (sizeof(cplx) + sizeof(double) + sizeof(int)) + sizeof(HouseShared<cplx, kHessWarps>) +
+      sizeof(SweepShared) + 1024;
   if (hb + static_smem <= (size_t)optin) {
     a->hess_smem = hb;
   } else {
