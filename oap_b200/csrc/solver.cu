@@ -54,7 +54,7 @@
 namespace oapb {
 
 constexpr int kGsThreads = 256;
-constexpr int kUpdThreads = 256;
+constexpr int kUpdRows = 64, kUpdGroups = 4, kUpdThreads = kUpdRows * kUpdGroups;
 
 // ------------------------------------------------------------ vector kernels
 __global__ void k_init_vector(double* fre, double* fim, int n, uint64_t seed, int mode) {
@@ -121,6 +121,7 @@ template <bool CPLX>
 __global__ void k_normalize(const double* __restrict__ fre, const double* __restrict__ fim, int n,
                             const DevState* st, double* vre, double* vim, float* x32re, float* x32im, cplx* H,
                             int m, int j, DevState* wst) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   const double beta = sqrt(st->fnorm2);
   const double inv = beta > 0 ? 1.0 / beta : 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -152,6 +153,7 @@ template <bool CPLX>
 __global__ void __launch_bounds__(1024)
 k_breakdown_fix(const double* __restrict__ Vre, const double* __restrict__ Vim, int n, int j, double* fre,
                 double* fim, DevState* st, uint64_t seed) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   const double f2 = st->fnorm2, scale2 = st->hnorm2 + st->fnorm2;
   if (threadIdx.x == 0) st->brk = 0;
   if (!(f2 <= 1e-24 * scale2)) return;
@@ -232,6 +234,7 @@ __global__ void __launch_bounds__(kGsThreads)
 k_gs_project(const double* __restrict__ Vre, const double* __restrict__ Vim, int n, int nvec,
              const double* __restrict__ xre, const double* __restrict__ xim, int chunk, cplx* part, int ldp,
              const DevState* st, int gated) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   if (gated && !st->dgks) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long r0 = (long)blockIdx.x * chunk;
@@ -259,6 +262,7 @@ k_gs_project(const double* __restrict__ Vre, const double* __restrict__ Vim, int
 // coef[i] = sum_b part[b][i]   (one block)
 __global__ void k_gs_reduce(const cplx* part, int nblk, int ldp, int nvec, cplx* coef, const DevState* st,
                             int gated) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   if (gated && !st->dgks) return;
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
     double a = 0, b = 0;
@@ -271,32 +275,58 @@ __global__ void k_gs_reduce(const cplx* part, int nblk, int ldp, int nvec, cplx*
   }
 }
 
-// f = src - sum_i V_i coef[i]; fpart[b] = block's share of ||f||^2
+// f = src - sum_i V_i coef[i]; fpart[b] = block's share of ||f||^2.  Four
+// threads per row take a quarter of the vectors each, added in order: a thread's
+// loads over i are the kernel's latency, and at n = 4096 one thread per row
+// fills 16 blocks only.  With the step's kernels as dependent launches: 96 steps
+// of the implicit Gram operator, 4096 x 65536, 51.3 -> 48.1 ms a solve, 581 x
+// 7813 (m = 65) 6.6 -> 5.0.
 template <bool CPLX>
 __global__ void __launch_bounds__(kUpdThreads)
 k_gs_update(const double* __restrict__ Vre, const double* __restrict__ Vim, int n, int nvec, const cplx* coef,
             const double* srcre, const double* srcim, double* fre, double* fim, double* fpart,
             const DevState* st, int gated) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   if (gated && !st->dgks) return;
   __shared__ cplx c[kMaxM + 1];
+  __shared__ double pr[kUpdGroups][kUpdRows], pi[CPLX ? kUpdGroups : 1][kUpdRows];
   for (int i = threadIdx.x; i < nvec; i += blockDim.x) c[i] = coef[i];
   __syncthreads();
+  const int row = threadIdx.x % kUpdRows, g = threadIdx.x / kUpdRows;
+  const int i0 = nvec * g / kUpdGroups, i1 = nvec * (g + 1) / kUpdGroups;
   double s = 0;
-  for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
-    double ar = srcre[r], ai = CPLX ? srcim[r] : 0.0;
-    for (int i = 0; i < nvec; ++i) {
-      double vr = Vre[(long)i * n + r];
-      if (CPLX) {
-        double vi = Vim[(long)i * n + r];
-        ar -= vr * c[i].re - vi * c[i].im;
-        ai -= vr * c[i].im + vi * c[i].re;
-      } else {
-        ar -= vr * c[i].re;
+  for (long base = (long)blockIdx.x * kUpdRows; base < n; base += (long)gridDim.x * kUpdRows) {
+    const long r = base + row;
+    double ar = 0, ai = 0;
+    if (r < n) {
+#pragma unroll 8
+      for (int i = i0; i < i1; ++i) {
+        double vr = Vre[(long)i * n + r];
+        if (CPLX) {
+          double vi = Vim[(long)i * n + r];
+          ar += vr * c[i].re - vi * c[i].im;
+          ai += vr * c[i].im + vi * c[i].re;
+        } else {
+          ar += vr * c[i].re;
+        }
       }
     }
-    fre[r] = ar;
-    if (CPLX) fim[r] = ai;
-    s += ar * ar + ai * ai;
+    pr[g][row] = ar;
+    if (CPLX) pi[g][row] = ai;
+    __syncthreads();
+    if (g == 0 && r < n) {
+      ar = srcre[r];
+      ai = CPLX ? srcim[r] : 0.0;
+#pragma unroll
+      for (int q = 0; q < kUpdGroups; ++q) {
+        ar -= pr[q][row];
+        if (CPLX) ai -= pi[q][row];
+      }
+      fre[r] = ar;
+      if (CPLX) fim[r] = ai;
+      s += ar * ar + ai * ai;
+    }
+    __syncthreads();
   }
   __shared__ double red[32];
   s = warp_sum(s);
@@ -313,6 +343,7 @@ k_gs_update(const double* __restrict__ Vre, const double* __restrict__ Vim, int 
 // pass is needed.  pass 1: h += s, write H[:, j].  Zeroes H below the column.
 __global__ void k_gs_finalize(const double* fpart, int np, cplx* h, const cplx* s, cplx* H, int m, int j,
                               double rho, DevState* st, int pass, int real_basis) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // dependent launch
   if (pass == 1 && !st->dgks) return;
   const double f2 = block_sum(fpart, np);
   const int nvec = j + 1;
@@ -641,13 +672,13 @@ int gs_pass(oapb_arnoldi* a, int j, const double* srcre, const double* srcim, cp
   cudaStream_t s = a->stream;
   const int n = a->n, nvec = j + 1;
   ++a->stats.kernel_launches;
-  k_gs_project<C><<<a->nchunk, kGsThreads, 0, s>>>(a->Vre, a->Vim, n, nvec, srcre, srcim, a->chunk, a->part,
-                                                    a->m + 1, a->st, gated);
+  launch_dependent(k_gs_project<C>, dim3(a->nchunk), dim3(kGsThreads), 0, s, a->Vre, a->Vim, n, nvec, srcre, srcim,
+                   a->chunk, a->part, a->m + 1, a->st, gated);
   ++a->stats.kernel_launches;
-  k_gs_reduce<<<1, 128, 0, s>>>(a->part, a->nchunk, a->m + 1, nvec, coef, a->st, gated);
+  launch_dependent(k_gs_reduce, dim3(1), dim3(128), 0, s, a->part, a->nchunk, a->m + 1, nvec, coef, a->st, gated);
   ++a->stats.kernel_launches;
-  k_gs_update<C><<<a->nupd, kUpdThreads, 0, s>>>(a->Vre, a->Vim, n, nvec, coef, srcre, srcim, a->fre, a->fim,
-                                                 a->fpart, a->st, gated);
+  launch_dependent(k_gs_update<C>, dim3(a->nupd), dim3(kUpdThreads), 0, s, a->Vre, a->Vim, n, nvec, coef, srcre, srcim,
+                   a->fre, a->fim, a->fpart, a->st, gated);
   return launch_check();
 }
 
@@ -659,11 +690,11 @@ int arnoldi_step(oapb_arnoldi* a, int j, bool fp32) {
   double* vim = C ? a->Vim + (long)j * n : nullptr;
   if (j > 0) ++a->stats.kernel_launches;
   if (j > 0)
-    k_breakdown_fix<C><<<1, 1024, 0, s>>>(a->Vre, a->Vim, n, j, a->fre, a->fim, a->st,
-                                          a->cfg.seed * 7919ull + (uint64_t)(a->stats.restarts * 1024 + j));
+    launch_dependent(k_breakdown_fix<C>, dim3(1), dim3(1024), 0, s, a->Vre, a->Vim, n, j, a->fre, a->fim, a->st,
+                     a->cfg.seed * 7919ull + (uint64_t)(a->stats.restarts * 1024 + j));
   ++a->stats.kernel_launches;
-  k_normalize<C><<<grid_n(n), 256, 0, s>>>(a->fre, a->fim, n, a->st, vre, vim, fp32 ? a->x32re : nullptr,
-                                           fp32 ? a->x32im : nullptr, a->H, m, j, a->st);
+  launch_dependent(k_normalize<C>, dim3(grid_n(n)), dim3(256), 0, s, a->fre, a->fim, n, a->st, vre, vim,
+                   fp32 ? a->x32re : nullptr, fp32 ? a->x32im : nullptr, a->H, m, j, a->st);
   int rc = launch_check();
   if (rc) return rc;
   rc = apply_op(a, vre, vim, a->wre, a->wim, fp32, OAPB_TYPE_WV);
@@ -676,10 +707,12 @@ int arnoldi_step(oapb_arnoldi* a, int j, bool fp32) {
   // rho rule leaves 1e-6 of orthogonality on image spectra, and H then fails
   // the symmetry check (a general eigensolve at m = 96 took 20 ms)
   const double rho = (a->gX || a->gS) ? 1e300 : a->cfg.rho;
-  k_gs_finalize<<<1, 256, 0, s>>>(a->fpart, a->nupd, a->h, a->s, a->H, m, j, rho, a->st, 0, !C);
+  launch_dependent(k_gs_finalize, dim3(1), dim3(256), 0, s, a->fpart, a->nupd, a->h, a->s, a->H, m, j, rho, a->st, 0,
+                   !C);
   if ((rc = gs_pass<C>(a, j, a->fre, a->fim, a->s, 1))) return rc;
   ++a->stats.kernel_launches;
-  k_gs_finalize<<<1, 256, 0, s>>>(a->fpart, a->nupd, a->h, a->s, a->H, m, j, a->cfg.rho, a->st, 1, !C);
+  launch_dependent(k_gs_finalize, dim3(1), dim3(256), 0, s, a->fpart, a->nupd, a->h, a->s, a->H, m, j, a->cfg.rho,
+                   a->st, 1, !C);
   return launch_check();
 }
 
@@ -1877,7 +1910,7 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
     a->nchunk = 2 * kNumSMs;
     a->chunk = (n + a->nchunk - 1) / a->nchunk;
   }
-  a->nupd = grid_for(n, kUpdThreads, kNumSMs * 4);
+  a->nupd = grid_for(n, kUpdRows, kNumSMs * 4);
   int rc = OAPB_OK;
   const bool C = a->is_c;
   rc |= dalloc(&a->Vre, vb * (m + 1));
