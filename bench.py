@@ -779,8 +779,8 @@ def c4_result():
             "matvecs": stats["matvecs"], "restarts": stats["restarts"],
             "roofline": {"bound": "hbm", "algorithmic_bytes": stats["operator_bytes"], "achieved_GBs": gbs,
                          "peak": hbm, "frac": gbs / hbm,
-                         "note": "operator bytes of every matvec (16 n^2 each, complex) over the launch time; the "
-                                 "problems in flight exceed L2, so each matvec streams its operator from HBM"},
+                         "note": "operator bytes of every pass (16 n^2 each, complex) over the launch time; the "
+                                 "problems in flight exceed L2, so each pass streams its operator from HBM"},
             "problems": len(sizes), "max_residual": float(res.max()),
             "eig_err_vs_plain_fp64_sample8": err}
 
