@@ -225,8 +225,8 @@ static __device__ int find_split(const Cx* T, int ld, int h, int lane) {
 // Clocks per rotation at m = 32, FP64 (FP32): one warp, the window normalised
 // before its products and the column rotations of T and Z after the chain, 457
 // + 265 (323 + 211); now 334 + 112 (197 + 72), at m = 64 413 + 104 before 582 +
-// 487.  A Schur form with 24 exact shifts, m = 32: 1114 -> 720 us (714 -> 395);
-// m = 64, 56 shifts: 6.13 -> 3.06 ms (3.93 -> 1.58).  An FP64 instruction holds
+// 487.  A Schur form with 24 exact shifts, m = 32: 1097 -> 715 us (684 -> 392);
+// m = 64, 56 shifts: 6.05 -> 3.00 ms (4.00 -> 1.67).  An FP64 instruction holds
 // a warp's FP64 port for about 4 clocks: the chain's 80 are what bounds it.
 // (Column rotations of T inside the chain's loop, a step behind it, made that
 // 512 clocks per rotation.)
