@@ -1939,7 +1939,6 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
     rc |= dalloc(&a->cbar, sizeof(unsigned));
   }
   const size_t hb = sizeof(cplx) * hess_ws_cplx(m);
-  const size_t hb_block = sizeof(cplx) * hess_ws_cplx(kBmMaxB);  // small_eig of the block methods
   int dev = 0, optin = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1958,18 +1957,16 @@ int oapb_arnoldi_create(oapb_arnoldi** out, const oapb_arnoldi_config* cfg, void
   } else {
     rc |= dalloc(&a->hws, hb);
   }
-  {
-    const size_t attr = std::max(a->hess_smem, hb_block);
-    if (attr > 48 * 1024 &&
-        cudaFuncSetAttribute(k_hess, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attr) != cudaSuccess)
-      rc |= OAPB_ERR_CUDA;
-  }
-  // (k_vq takes m x (kept vectors + 1) or m x (k + 4) coefficients)
-  const size_t vqb = std::min(sizeof(cplx) * (size_t)m * (size_t)std::min(m, std::max(restart_keep(m, k, false), k + 3) + 1), (size_t)optin);
-  if (vqb > 48 * 1024) {
-    cudaFuncSetAttribute(k_vq<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vqb);
-    cudaFuncSetAttribute(k_vq<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vqb);
-  }
+  // The dynamic shared-memory limit belongs to the kernel on the device, and
+  // handles of other sizes set it too: always the most these kernels can take,
+  // so that no later handle lowers it below what an earlier one launches with.
+  // (k_hess also runs the block methods' eigenproblem of up to kBmMaxB vectors;
+  // k_vq takes m x the vectors it forms)
+  if (cudaFuncSetAttribute(k_hess, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)static_smem) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_vq<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
+      cudaFuncSetAttribute(k_vq<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess)
+    rc |= OAPB_ERR_CUDA;
   if (rc != OAPB_OK) {
     free_all(a);
     if (a->own_stream) cudaStreamDestroy(a->stream);

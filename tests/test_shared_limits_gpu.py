@@ -1,0 +1,71 @@
+"""Handles and host threads that use the same kernels with different dynamic
+shared-memory sizes: what one sets does not refuse another's launch."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+import oap_b200 as B  # noqa: E402
+
+TOL = 1e-10
+
+
+def operator(n, seed, k):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    A = torch.randn(n, n, dtype=torch.float64, device="cuda", generator=g)
+    A = (A + A.T) / (2 * n ** 0.5)
+    i = torch.arange(k, device="cuda")
+    A[i, i] += 4.0 + 0.05 * i.double()
+    return A.contiguous()
+
+
+def dense(m, k, cplx, per_step):
+    n = 3 * m + 40
+    A = operator(n, m, k)
+    s = B.Arnoldi(n, m, k, is_complex=cplx, tolerance=TOL, seed=3, autotune=2 if per_step else True)
+    s.set_operator(A, torch.zeros_like(A) if cplx else None)
+    return s, A
+
+
+def gram(m, k):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m)
+    rows, cols = 3 * m + 12, 640
+    U = torch.randn(rows, k, generator=g, device="cuda") * torch.linspace(9.0, 6.0, k, device="cuda")
+    X = (U @ torch.randn(k, cols, generator=g, device="cuda") / cols ** 0.5
+         + 0.02 * torch.randn(rows, cols, generator=g, device="cuda")).contiguous()
+    s = B.Arnoldi(rows, m, k, tolerance=TOL, seed=3)
+    s.set_gram_operator(X)
+    Xd = X.double()
+    return s, Xd @ Xd.T
+
+
+# the larger handle first, then one of a smaller Krylov space: the basis
+# products (m x vectors formed) and the small eigenproblem's workspace, on the
+# one-launch cycles and the per-step kernels
+@pytest.mark.parametrize("big,small,cplx,per_step", [((128, 60), (96, 32), False, False), ((128, 60), (96, 32), False, True),
+                                                     ((64, 8), (20, 4), False, False), ((64, 40), (40, 8), True, True),
+                                                     ((100, 50), (64, 46), True, False)])
+def test_handle_after_a_smaller_one(big, small, cplx, per_step):
+    pairs = [dense(*mk, cplx, per_step) for mk in (big, small)]
+    for (s, A), (_, k) in zip(pairs, (big, small)):
+        ev, res, st = s.solve()
+        assert st == B.OK and max(res) <= TOL
+        # eigenvalues of a symmetric operator: residuals <= 1e-10 leave rounding
+        ref = torch.linalg.eigvalsh(A).cpu().numpy()
+        ref = ref[np.argsort(-np.abs(ref))][:k]
+        assert np.abs(np.sort(np.array(ev).real) - np.sort(ref)).max() <= A.shape[0] * 2.3e-16 * 4 * np.abs(ref).max()
+
+
+def test_gram_handle_after_a_smaller_one():
+    pairs = [gram(96, 32), gram(64, 45)]
+    for (s, G), k in zip(pairs, (32, 45)):
+        ev, res, st = s.solve()
+        assert st == B.OK and max(res) <= TOL
+        ref = torch.linalg.eigvalsh(G).flip(0)[:k].cpu().numpy()
+        assert np.abs(np.array(ev).real - ref).max() <= (G.shape[0] + 640) * 2.3e-16 * 4 * ref[0]
