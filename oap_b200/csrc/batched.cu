@@ -387,6 +387,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
   __syncthreads();
   int start = 0;
   for (int rs = 0; status == OAPB_OK; ++rs) {
+    const bool spike = rs > 0 && S.st->spike;
     for (int j = start; j < m; ++j) {
       // invariant-subspace breakdown: new random direction orthogonal to V
       bool brk = false;
@@ -419,7 +420,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
         }
       }
       if (tid == 0 && j > 0) {
-        if (!(rs > 0 && j == start && S.st->spike))  // else row j of H is already there
+        if (!(spike && j == start))  // else row j of H is already there
           S.H[j + (j - 1) * m] = cplx{brk ? 0.0 : beta, 0};
         else if (brk)
           for (int i = 0; i < j; ++i) S.H[j + i * m] = cplx{0, 0};
@@ -435,7 +436,7 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       double h2 = 0;
       for (int i = 0; i <= j; ++i) h2 += abs2(S.h[i]);
       hnorm2 = h2;
-      if (sqrt(fnorm2) < A.rho * sqrt(hnorm2)) {  // DGKS (ArnoldiProcedures.cpp:446-456)
+      if (sqrt(fnorm2) < dgks_rho(A.rho, spike, start, j) * sqrt(hnorm2)) {  // DGKS (ArnoldiProcedures.cpp:446-456)
         cta_project<C, NT>(Vr, Vi, n, j + 1, S.fr, S.fi, S.s);
         __syncthreads();
         fnorm2 = cta_update<C, NT>(Vr, Vi, n, j + 1, S.s, S.fr, S.fi, S.fr, S.fi, S.red);

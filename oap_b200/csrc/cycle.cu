@@ -500,7 +500,7 @@ struct Cycle {
       if (!project(S.wr, S.wi, j + 1, S.h)) return false;
       hn2 = sum_h2(j + 1);
       if (!update(S.wr, S.wi, j + 1, S.h, f2)) return false;
-      if (sqrt(f2) < a.rho * sqrt(hn2)) {  // DGKS (ArnoldiProcedures.cpp:446-456)
+      if (sqrt(f2) < dgks_rho(a.rho, spike, a.j0, j) * sqrt(hn2)) {  // DGKS (ArnoldiProcedures.cpp:446-456)
         ++dgks;
         if (!project(S.fr, S.fi, j + 1, S.s)) return false;
         if (!update(S.fr, S.fi, j + 1, S.s, f2)) return false;

@@ -355,7 +355,7 @@ __global__ void k_gs_finalize(const double* fpart, int np, cplx* h, const cplx* 
       hn = a;
     }
     __syncthreads();
-    const int dg = sqrt(f2) < rho * sqrt(hn);
+    const int dg = sqrt(f2) < dgks_rho(rho, st->spike, st->keep, j) * sqrt(hn);
     if (threadIdx.x == 0) {
       st->dgks = dg;
       st->hnorm2 = hn;
