@@ -421,8 +421,12 @@ static int max_clusters(K kern, const GramFusedPlan& p, size_t smem) {
 template <int LPR, bool SHIFT, bool FULL>
 static int gram_fused(const GramFusedPlan& p, GramFusedArgs g, double* w, bool accumulate, cudaStream_t s) {
   auto kern = k_gram_fused<LPR, SHIFT, FULL>;
-  const size_t smem = sizeof(float) * kGfStages * (size_t)(kGfThreads / LPR) * p.rpt * gf_pitch(LPR, SHIFT);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  constexpr size_t row_group = sizeof(float) * kGfStages * (kGfThreads / LPR) * gf_pitch(LPR, SHIFT);
+  const size_t smem = row_group * p.rpt;
+  // the limit is the kernel's, shared with every other thread's launches: always
+  // what the most rows per thread take
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(row_group * kGfRows)) !=
+      cudaSuccess)
     return OAPB_ERR_CUDA;
   g.clusters = std::min(max_clusters(kern, p, smem), (g.cols + 4 * LPR - 1) / (4 * LPR));
   cudaLaunchAttribute at;

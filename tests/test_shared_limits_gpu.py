@@ -1,5 +1,7 @@
 """Handles and host threads that use the same kernels with different dynamic
 shared-memory sizes: what one sets does not refuse another's launch."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -69,3 +71,44 @@ def test_gram_handle_after_a_smaller_one():
         assert st == B.OK and max(res) <= TOL
         ref = torch.linalg.eigvalsh(G).flip(0)[:k].cpu().numpy()
         assert np.abs(np.array(ev).real - ref).max() <= (G.shape[0] + 640) * 2.3e-16 * 4 * ref[0]
+
+
+def in_threads(work, count):
+    """work(i) on `count` host threads at once; the first exception is raised here."""
+    errors = []
+
+    def run(i):
+        try:
+            work(i)
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(count)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    if errors:
+        raise errors[0]
+
+
+def test_gram_operators_on_host_threads():
+    # row counts that share an instance of the kernel with other rows per thread
+    rows = (2000, 300, 1100, 2000)
+    handles = []
+    for i, r in enumerate(rows):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(i)
+        X = torch.randn(r, 640, device="cuda", generator=g)
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        s = B.Arnoldi(r, 24, 4, seed=3, max_restarts=6, stream=stream.cuda_stream)
+        s.set_gram_operator(X)
+        handles.append((s, stream, s.solve(allow_not_converged=True)))
+
+    def work(i):
+        s, _, ref = handles[i]
+        for _ in range(60):
+            assert s.solve(allow_not_converged=True) == ref  # the same launches: the same bits
+
+    in_threads(work, len(rows))
