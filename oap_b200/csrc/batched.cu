@@ -753,7 +753,9 @@ int oapb_arnoldi_solve_batched(const oapb_arnoldi_config* cfg, const oapb_batch_
   int gmax = 0;
   for (int v = 0; v < kBtVariants; ++v) {
     const void* kern = batched_kernel(v);
-    OAPB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // (the limit is the kernel's, shared with the calls of other threads: always
+    // the most a call may take)
+    OAPB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     int occ = 0;
     OAPB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kBtThreadsOf[v], smem));
     grids[v] = std::min(kNumSMs * occ, (int)count);

@@ -633,7 +633,10 @@ int launch_block_matvec_i8(const I8Operator& op, const double* xr, const double*
   if (g.stages < 2) return OAPB_ERR_ARG;
   const size_t smem = g.stages * stage + 1024;
   auto kern = cplx ? k_block_matvec_i8<true> : k_block_matvec_i8<false>;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  // (the limit is the kernel's, shared with the launches of other threads: the
+  // same for every block width)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kI8SmemBudget + 1024)) !=
+      cudaSuccess)
     return OAPB_ERR_CUDA;
   if (kev) cudaEventRecord(kev[0], s);
   if (launch_dependent(kern, dim3(g.grid.grid), dim3(kI8Threads), smem, s, g) != cudaSuccess) return OAPB_ERR_CUDA;

@@ -501,7 +501,10 @@ int launch_block_matvec_tc(const BtcOperator& op, const double* xr, const double
   auto kern = bf16_only ? (xlo ? (cplx ? k_block_matvec_tc<true, false, true> : k_block_matvec_tc<false, false, true>)
                               : (cplx ? k_block_matvec_tc<true, false, false> : k_block_matvec_tc<false, false, false>))
                         : (cplx ? k_block_matvec_tc<true, true, true> : k_block_matvec_tc<false, true, true>);
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  // (the limit is the kernel's, shared with the launches of other threads: the
+  // same for every block width)
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBtcSmemBudget + 1024)) !=
+      cudaSuccess)
     return OAPB_ERR_CUDA;
   if (kev) cudaEventRecord(kev[0], s);
   if (launch_dependent(kern, dim3(g.grid.grid), dim3(kBtcThreads), smem, s, g) != cudaSuccess) return OAPB_ERR_CUDA;

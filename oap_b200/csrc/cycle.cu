@@ -553,8 +553,9 @@ int device_limits(int* sms, int* optin) {
 template <bool C, bool RES, bool VEC>
 int launch(const CyclePlan& p, const CycleArgs& a, cudaStream_t s) {
   const void* k = (const void*)k_arnoldi_cycle<C, RES, VEC>;
-  if (p.smem > 48 * 1024 &&
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem) != cudaSuccess)
+  // (the limit is the kernel's, shared with the launches of other handles:
+  // always the same)
+  if (p.smem > 48 * 1024 && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, p.limit) != cudaSuccess)
     return OAPB_ERR_CUDA;
   CycleArgs args = a;
   int rows = p.rows, segs = p.segs;
@@ -569,6 +570,7 @@ int launch(const CyclePlan& p, const CycleArgs& a, cudaStream_t s) {
 bool cycle_plan(int n, int m, bool cplx, CyclePlan* p) {
   int sms = 0, optin = 0;
   if (m > kCyMaxM || device_limits(&sms, &optin)) return false;
+  p->limit = optin;
   // at least eight rows per CTA: below that a CTA's share of the products is
   // shorter than what its arrival at the barriers costs
   int g = std::min(sms, (n + 7) / 8);

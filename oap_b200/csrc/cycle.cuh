@@ -35,6 +35,7 @@ struct CyclePlan {
   int ctas = 0, rows = 0, segs = 1;
   bool resident = false;
   size_t smem = 0;
+  int limit = 0;  // the device's shared memory per CTA
 };
 
 // false where the per-step kernels run instead: x, the basis rows and the

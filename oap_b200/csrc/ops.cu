@@ -339,7 +339,8 @@ static int prep_ws(const void* kernel, size_t bytes, cudaStream_t s, Scratch& w)
   if (bytes + 1024 <= smem_limit()) {
     w.shm = bytes;
     if (bytes > 48 * 1024)
-      OAPB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+      // (the limit is the kernel's, shared with other threads' launches)
+      OAPB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_limit() - 1024));
   } else {
     OAPB_CUDA_TRY(cudaMallocAsync(&w.g, bytes, s));
   }

@@ -112,3 +112,75 @@ def test_gram_operators_on_host_threads():
             assert s.solve(allow_not_converged=True) == ref  # the same launches: the same bits
 
     in_threads(work, len(rows))
+
+
+def test_batched_solves_on_host_threads():
+    shapes = [(40, 32, 512, 32), (60, 24, 40, 8), (40, 200, 300, 24), (60, 16, 24, 6)]  # problems, sizes, hdim
+    sets = []
+    for i, (count, lo, hi, hdim) in enumerate(shapes):
+        rng = np.random.default_rng(i)
+        sets.append(([(operator(int(n), 100 * i + j, 3), None) for j, n in enumerate(rng.integers(lo, hi + 1, count))], hdim))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in shapes]
+
+    def solve(i):
+        mats, hdim = sets[i]
+        ev, res, st, _, _ = B.solve_batched(mats, 2, hdim=hdim, max_restarts=50, stream=streams[i].cuda_stream)
+        return ev, res, st
+
+    refs = [solve(i) for i in range(len(shapes))]
+
+    def work(i):
+        for _ in range(30):
+            for a, b in zip(solve(i), refs[i]):
+                assert np.array_equal(a, b)
+
+    in_threads(work, len(shapes))
+
+
+def test_block_passes_on_host_threads():
+    # block widths of other stage counts and sizes on the tensor-core passes
+    n = 1024
+    widths = (4, 32, 12, 24)
+    todo = []
+    for i, b in enumerate(widths):
+        A = operator(n, i, 3)
+        stream = torch.cuda.Stream()
+        torch.cuda.synchronize()
+        s = B.Arnoldi(n, 24, 4, precision=B.PREC_MIXED, stream=stream.cuda_stream)
+        s.set_operator(A)
+        X = torch.randn(b, n, dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(b))
+        ref = X @ A.T
+        torch.cuda.synchronize()
+        todo.append((s, ref, X, stream, n ** 0.5 * A.abs().max().item() * X.abs().max().item()))
+
+    def work(i):
+        s, ref, X, stream, scale = todo[i]
+        for _ in range(60):
+            # FP64-class slices: 2^-42 of each row's scale and FP32-class planes:
+            # 2^-15 per product, the sums of n growing like sqrt(n)
+            for precision, tol in ((B.PREC_FP64, 2.0 ** -42), (B.PREC_MIXED, 2.0 ** -15)):
+                with torch.cuda.stream(stream):
+                    W, _ = s.apply_block(X, precision=precision)
+                    err = (W - ref).abs().max().item()
+                assert err <= tol * scale
+
+    in_threads(work, len(widths))
+
+
+def test_qr_on_host_threads():
+    sizes = (60, 70, 56, 65)
+    mats = [operator(n, n, 2) for n in sizes]
+    streams = [torch.cuda.Stream() for _ in sizes]
+    torch.cuda.synchronize()
+
+    def work(i):
+        n, A = sizes[i], mats[i]
+        with torch.cuda.stream(streams[i]):
+            Q, R = torch.empty_like(A), torch.empty_like(A)
+            for _ in range(200):
+                a, q, r = B.mat(A), B.mat(Q), B.mat(R)
+                B.check(B.lib().oapb_qr_givens(q, r, a, streams[i].cuda_stream), "oapb_qr_givens")
+            assert (Q @ R - A).abs().max().item() <= 8 * n * 2.3e-16 * A.abs().max().item()
+
+    in_threads(work, len(sizes))
