@@ -164,6 +164,16 @@ OAPB_EXPORT int oapb_calc_triangular_h(const oapb_mat* H, const oapb_mat* Q,
 OAPB_EXPORT int oapb_selftest_bounded_wait(uint32_t limit_us, int32_t arrive, int32_t* timed_out,
                                            void* stream);
 
+/* Self-test of the implicit Gram operator's exchange between the CTAs of a
+ * cluster when one of them is late (no counterpart in the reference).  The last
+ * CTA pauses for three limits before it sends its sums of panel `late` (0 .. 15;
+ * -1: no pause): its peers' waits of limit_us microseconds (1 .. 100000) run
+ * out, they stay until it has left too, and the call returns OAPB_ERR_TIMEOUT
+ * with *timed_out = 1; without the pause OAPB_OK and *timed_out = 0.  The context
+ * stays usable either way.  Synchronises `stream`. */
+OAPB_EXPORT int oapb_selftest_gram_wait(uint32_t limit_us, int32_t late, int32_t* timed_out,
+                                        void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Solver: CuHArnoldi / CuHArnoldiCallback (ArnoldiPackage)                  */
 /* ------------------------------------------------------------------------ */

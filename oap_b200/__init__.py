@@ -119,6 +119,7 @@ def lib():
             "oapb_qr_householder": [P(Mat), P(Mat), P(Mat), vp],
             "oapb_qr_givens_noalloc": [P(Mat), P(Mat), P(Mat), vp],
             "oapb_selftest_bounded_wait": [C.c_uint32, C.c_int32, P(C.c_int32), vp],
+            "oapb_selftest_gram_wait": [C.c_uint32, C.c_int32, P(C.c_int32), vp],
             "oapb_arnoldi_set_gram_operator_host": [vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint64],
             "oapb_arnoldi_gram_stream_info": [vp, P(C.c_uint32), P(C.c_uint32), P(C.c_uint64)],
             "oapb_is_upper_triangular": [P(C.c_int), P(Mat), C.c_double, vp],
@@ -395,6 +396,14 @@ def selftest_bounded_wait(limit_us, arrive=False, stream=None):
     returns (status, timed_out).  arrive=False lets the wait run out."""
     out = C.c_int32(-1)
     st = lib().oapb_selftest_bounded_wait(int(limit_us), int(bool(arrive)), C.byref(out), _stream(stream))
+    return st, out.value
+
+
+def selftest_gram_wait(limit_us, late=-1, stream=None):
+    """Run the Gram operator's late-CTA self-test (oapb_selftest_gram_wait):
+    returns (status, timed_out).  late: the panel whose sums come late, -1 none."""
+    out = C.c_int32(-1)
+    st = lib().oapb_selftest_gram_wait(int(limit_us), int(late), C.byref(out), _stream(stream))
     return st, out.value
 
 

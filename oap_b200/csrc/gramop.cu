@@ -131,16 +131,28 @@ struct GramFusedArgs {
   const double* v;
   double* part;  // clusters x rows
   int rows, cols, rpt, cluster, clusters;
+  unsigned long long limit_ns;  // of every wait
+  int late;  // self-test: the panel before whose sums the last CTA pauses for three limits
 };
 
 // t's exchange: each CTA writes its sums to every CTA of the cluster with
 // st.async, counted by an mbarrier there.  (A cluster barrier would do, but its
 // release waits for the panel copies in flight: a third of all issue slots.)
 // A wait that runs out (2 s) ends the CTA with NaN sums, which the solver
-// reports.
+// reports.  Its peers may still send it theirs, so it stays until each of them
+// has left too (which they do when they have every sum, or when they miss its
+// next one) and, for the sums a late peer sent last, until these have arrived or
+// kGfDrainNs have passed.
 constexpr unsigned long long kGfLimitNs = 2000000000ull;
+constexpr unsigned long long kGfDrainNs = 1000000ull;
 
-__device__ __forceinline__ bool gf_wait(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ unsigned long long gf_now() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+__device__ __forceinline__ bool gf_wait(uint32_t bar, uint32_t parity, unsigned long long limit_ns) {
   unsigned long long t0 = 0;
   for (unsigned it = 0;; ++it) {
     uint32_t done;
@@ -152,10 +164,9 @@ __device__ __forceinline__ bool gf_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     if (done) return true;
     if ((it & 63u) == 63u) {
-      unsigned long long t;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+      const unsigned long long t = gf_now();
       if (!t0) t0 = t;
-      if (t - t0 > kGfLimitNs) return false;
+      if (t - t0 > limit_ns) return false;
     }
   }
 }
@@ -167,8 +178,8 @@ __device__ __forceinline__ void gf_copy(uint32_t dst, const void* src, int bytes
 
 __host__ __device__ constexpr int gf_pitch(int lpr, bool shift) { return 4 * lpr + (shift ? 4 : 0); }
 
-// FULL: every thread has kGfRows rows, all inside the matrix
-template <int LPR, bool SHIFT, bool FULL>
+// FULL: every thread has kGfRows rows, all inside the matrix.  TEST: g.late holds
+template <int LPR, bool SHIFT, bool FULL, bool TEST = false>
 __global__ void __launch_bounds__(kGfThreads, 2) k_gram_fused(GramFusedArgs g) {
   constexpr int W = 4 * LPR, RG = kGfThreads / LPR, NW = kGfThreads / 32, P = gf_pitch(LPR, SHIFT);
   extern __shared__ __align__(16) float xs[];  // stages x (RG rpt) x P
@@ -235,7 +246,8 @@ __global__ void __launch_bounds__(kGfThreads, 2) k_gram_fused(GramFusedArgs g) {
   load(0);
   load(1);
   bool ok = true;
-  for (int i = 0; i < iters; ++i) {
+  int i = 0;
+  for (; i < iters; ++i) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kGfStages - 1) : "memory");
     if (SHIFT) __syncthreads();
     const float* x = xs + (i % kGfStages) * stage;
@@ -297,6 +309,9 @@ __global__ void __launch_bounds__(kGfThreads, 2) k_gram_fused(GramFusedArgs g) {
         ts[tid] = t;
       } else {
         const uint32_t at = gf_smem(&tp[i & 1][rank][tid]), bar = gf_smem(&bars[i & 1]);
+        if (TEST && i == g.late && rank == g.cluster - 1)
+          for (const unsigned long long t0 = gf_now(); gf_now() - t0 < 3 * g.limit_ns;) {
+          }
         if (tid == 0)
           asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                        "r"((uint32_t)(g.cluster * W * sizeof(double)))
@@ -309,7 +324,7 @@ __global__ void __launch_bounds__(kGfThreads, 2) k_gram_fused(GramFusedArgs g) {
                        "l"(__double_as_longlong(t)), "r"(tobar)
                        : "memory");
         }
-        ok = gf_wait(bar, (i >> 1) & 1);
+        ok = gf_wait(bar, (i >> 1) & 1, g.limit_ns);
         t = 0;
         for (int d = 0; d < g.cluster; ++d) t += tp[i & 1][d][tid];
         ts[tid] = t;
@@ -333,6 +348,11 @@ __global__ void __launch_bounds__(kGfThreads, 2) k_gram_fused(GramFusedArgs g) {
       for (int c = 0; c < 4; ++c) acc[j] = fma(xd[j][c], t[c], acc[j]);
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
+  if (!ok) {  // (only with a cluster)
+    asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;" ::: "memory");
+    gf_wait(gf_smem(&bars[i & 1]), (i >> 1) & 1, kGfDrainNs);
+    __syncthreads();
+  }
 #pragma unroll
   for (int j = 0; j < kGfRows; ++j)
     if (FULL || j < rpt) {
@@ -466,7 +486,7 @@ int launch_gram_apply(const float* X, int rows, int cols, const double* v, doubl
   if ((cols & 3) == 0 && ((uintptr_t)X & 15)) return OAPB_ERR_ARG;
   GramFusedPlan p;
   if (((uintptr_t)X & 15) == 0 && gram_fused_plan(rows, &p)) {
-    const GramFusedArgs g{X, v, ws, rows, cols, p.rpt, p.cluster, 0};
+    const GramFusedArgs g{X, v, ws, rows, cols, p.rpt, p.cluster, 0, kGfLimitNs, -1};
     switch (p.lpr) {
       case 16: return gram_fused_any<16>(p, g, w, accumulate, s);
       case 8: return gram_fused_any<8>(p, g, w, accumulate, s);
@@ -597,3 +617,36 @@ int gram_stream_resident_blocks(const GramStream* g) { return g ? g->resident : 
 int gram_stream_blocks(const GramStream* g) { return g ? g->nb : 0; }
 
 }  // namespace oapb
+
+using namespace oapb;
+
+extern "C" int oapb_selftest_gram_wait(uint32_t limit_us, int32_t late, int32_t* timed_out, void* stream) {
+  constexpr int kRows = 4096, kCols = 256;  // one cluster of 8 CTAs, 16 panels of 16 columns
+  if (!timed_out || limit_us == 0 || limit_us > 100000u || late < -1 || late >= kCols / 16) return OAPB_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  GramFusedPlan p;
+  if (!gram_fused_plan(kRows, &p) || p.lpr != 4 || p.rpt != kGfRows) return OAPB_ERR_ARG;
+  auto kern = k_gram_fused<4, false, true, true>;
+  const size_t smem = sizeof(float) * kGfStages * (kGfThreads / 4) * kGfRows * gf_pitch(4, false);
+  const size_t xb = sizeof(float) * kRows * kCols, vb = sizeof(double) * kRows;
+  char* buf = nullptr;
+  if (cudaMallocAsync((void**)&buf, xb + 2 * vb, s) != cudaSuccess) return OAPB_ERR_NOMEM;
+  static double part[kRows];
+  static std::mutex mu;  // of part
+  std::lock_guard<std::mutex> lock(mu);
+  const GramFusedArgs g{(const float*)buf, (const double*)(buf + xb), (double*)(buf + xb + vb),
+                        kRows, kCols, p.rpt, p.cluster, 1, (unsigned long long)limit_us * 1000ull, late};
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t cfg = gram_config(p, 1, smem, s, &at);
+  int rc = OAPB_OK;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+      cudaMemsetAsync(buf, 0, xb + 2 * vb, s) != cudaSuccess || cudaLaunchKernelEx(&cfg, kern, g) != cudaSuccess ||
+      cudaMemcpyAsync(part, g.part, vb, cudaMemcpyDeviceToHost, s) != cudaSuccess)
+    rc = OAPB_ERR_CUDA;
+  cudaFreeAsync(buf, s);
+  if (cudaStreamSynchronize(s) != cudaSuccess) rc = OAPB_ERR_CUDA;
+  if (rc) return rc;
+  *timed_out = 0;
+  for (double x : part) *timed_out |= x != x;
+  return *timed_out ? OAPB_ERR_TIMEOUT : OAPB_OK;
+}
