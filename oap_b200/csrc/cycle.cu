@@ -571,6 +571,7 @@ bool cycle_plan(int n, int m, bool cplx, CyclePlan* p) {
   int sms = 0, optin = 0;
   if (m > kCyMaxM || device_limits(&sms, &optin)) return false;
   p->limit = optin;
+  p->sms = sms;
   // at least eight rows per CTA: below that a CTA's share of the products is
   // shorter than what its arrival at the barriers costs
   int g = std::min(sms, (n + 7) / 8);

@@ -36,6 +36,7 @@ struct CyclePlan {
   bool resident = false;
   size_t smem = 0;
   int limit = 0;  // the device's shared memory per CTA
+  int sms = 0;    // and its SMs
 };
 
 // false where the per-step kernels run instead: x, the basis rows and the

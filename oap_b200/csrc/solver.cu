@@ -29,8 +29,10 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <map>
 #include <mutex>
+#include <optional>
 #include <tuple>
 #include <new>
 #include <stdio.h>
@@ -788,8 +790,45 @@ bool use_cycle(const oapb_arnoldi* a) {
 }
 
 // Two cooperative grids that each held part of the SMs would wait for one
-// another's CTAs: the restart loops of one process take turns.
-std::mutex g_cycle_mu;
+// another's CTAs.  A CTA takes one SM at most, so grids that together have no
+// more CTAs than the device has SMs always fit: a cycle waits, in order of
+// arrival, until the process's cycles under way on its device leave that much,
+// and gives it back at the check that follows it.  (One lock for every device
+// and whole solves made four threads with n = 100, 13 CTAs each, take four times
+// one's 1.1 ms.)
+struct CycleGate {
+  std::mutex mu;
+  std::condition_variable cv;
+  int used = 0;                  // CTAs of the cycles under way
+  uint64_t ticket = 0, turn = 0;  // order of arrival
+};
+CycleGate g_cycle_gates[64];  // per device
+
+class CycleSlot {
+ public:
+  explicit CycleSlot(const CyclePlan& p) : ctas_(p.ctas) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    gate_ = &g_cycle_gates[dev & 63];
+    std::unique_lock<std::mutex> lk(gate_->mu);
+    const uint64_t mine = gate_->ticket++;
+    gate_->cv.wait(lk, [&] { return gate_->turn == mine && gate_->used + ctas_ <= p.sms; });
+    gate_->used += ctas_;
+    ++gate_->turn;
+    gate_->cv.notify_all();
+  }
+  ~CycleSlot() {
+    std::lock_guard<std::mutex> lk(gate_->mu);
+    gate_->used -= ctas_;
+    gate_->cv.notify_all();
+  }
+  CycleSlot(const CycleSlot&) = delete;
+  CycleSlot& operator=(const CycleSlot&) = delete;
+
+ private:
+  CycleGate* gate_;
+  int ctas_;
+};
 
 // Steps start .. m - 1 in one launch; with `restarted`, the restart's V <- V Q
 // and f first.
@@ -824,18 +863,22 @@ template <bool C>
 int iram(oapb_arnoldi* a, bool fp32, double tol, unsigned max_restarts, int start) {
   DevState hs;
   const bool one = !fp32 && use_cycle(a);
-  std::unique_lock<std::mutex> turn(g_cycle_mu, std::defer_lock);
-  if (one) turn.lock();
   bool restarted = false;
   for (unsigned r = 0;; ++r) {
     int rc = OAPB_OK;
-    if (one && start < a->m) rc = cycle(a, start, restarted);
-    for (int j = start; !one && j < a->m && !rc; ++j) rc = arnoldi_step<C>(a, j, fp32);
-    if (rc) return rc;
     const int do_shift = r < max_restarts;
-    rc = hess(a, do_shift, tol);
+    {
+      std::optional<CycleSlot> slot;
+      if (one && start < a->m) {
+        slot.emplace(a->cyc);
+        rc = cycle(a, start, restarted);
+      }
+      for (int j = start; !one && j < a->m && !rc; ++j) rc = arnoldi_step<C>(a, j, fp32);
+      if (!rc) rc = hess(a, do_shift, tol);
+      if (!rc) rc = read_state(a, &hs);
+      if (rc && slot) cudaStreamSynchronize(a->stream);  // the slot outlives its cycle
+    }
     if (rc) return rc;
-    if ((rc = read_state(a, &hs))) return rc;
     if (hs.status & 4) return OAPB_ERR_NONFINITE;
     if (hs.status & 1) return OAPB_ERR_BREAKDOWN;
     if (hs.status & 2) return OAPB_ERR_TIMEOUT;
@@ -1646,13 +1689,25 @@ int finish_plain(oapb_arnoldi* a, int st, double* r) {
   return verify<C>(a, hs.scale, r);
 }
 
+// A solve that runs in cycles lets work already queued on its stream end before
+// it holds SMs back from the cycles of others (the solve waits for it anyway).
+int settle_stream(oapb_arnoldi* a) {
+  if (!use_cycle(a)) return OAPB_OK;
+  const cudaError_t e = cudaStreamQuery(a->stream);
+  if (e == cudaSuccess) return OAPB_OK;
+  if (e != cudaErrorNotReady) return OAPB_ERR_CUDA;
+  cudaGetLastError();
+  return cudaStreamSynchronize(a->stream) == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
+}
+
 // The plain FP64 GPU Arnoldi: IRAM to the goal, Ritz vectors, FP64
 // verification of every wanted pair in one block pass.
 template <bool C>
 int solve_plain(oapb_arnoldi* a, double* r) {
   a->nvec_hess = a->k;
-  int rc = iram_start<C>(a);
+  int rc = settle_stream(a);
   if (rc) return rc;
+  if ((rc = iram_start<C>(a))) return rc;
   int st = iram<C>(a, false, a->cfg.tolerance, a->cfg.max_restarts, 0);
   if (st == OAPB_NOT_CONVERGED && a->cfg.init == OAPB_INIT_USER && a->cfg.fallback_random) {
     // the warm start did not reach the goal: the random-start method decides
@@ -1669,9 +1724,10 @@ int solve_plain(oapb_arnoldi* a, double* r) {
 template <bool C>
 int resume_plain(oapb_arnoldi* a, double* r) {
   a->nvec_hess = a->k;
-  if (cudaMemsetAsync(a->st, 0, sizeof(DevState), a->stream) != cudaSuccess) return OAPB_ERR_CUDA;
-  int rc = set_fnorm(a);
+  int rc = settle_stream(a);
   if (rc) return rc;
+  if (cudaMemsetAsync(a->st, 0, sizeof(DevState), a->stream) != cudaSuccess) return OAPB_ERR_CUDA;
+  if ((rc = set_fnorm(a))) return rc;
   const int st = iram<C>(a, false, a->cfg.tolerance, a->cfg.max_restarts, a->m);
   return finish_plain<C>(a, st, r);
 }
