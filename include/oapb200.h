@@ -530,13 +530,15 @@ typedef struct oapb_batch_stats {
  * from a queue ordered by decreasing n and runs the full restart loop on the
  * device.  cfg: hdim caps the Krylov dimension (m_i = min(n_i, hdim),
  * hdim <= 32), wanted, sort, tolerance, max_restarts, rho, seed, autotune
- * (0: the default launch variant, 256 threads per CTA; 1: the variant
- * (threads per CTA x CTAs per SM the registers are budgeted for: 256 x 1,
- * 128 x 2, 256 x 2, 128 x 4, 64 x 8) of 256 x 2, 128 x 2 and 128 x 4 that ran
- * fastest on a sample of the first batch of a given largest n, hdim, wanted and
- * complexity, cached per device; 2 + v: variant v, 0..4); n, is_complex,
- * precision and init are ignored (complex iff im != NULL, FP64, seeded random
- * start).  `problems` is a HOST array.  Host outputs: eig_re / eig_im / residuals (count x wanted, row i = problem i in sort
+ * (0: the default launch variant, 256 threads per CTA; 1: of the variants
+ * (threads per CTA x CTAs per SM the registers are budgeted for) 256 x 1,
+ * 128 x 2, 256 x 2, 128 x 4 and 64 x 8 the one of the first four that ran
+ * fastest on a sample of the first batch of its kind (largest n to 64, hdim,
+ * wanted, complexity, problems to a power of two), cached per device, for
+ * batches of more problems than SMs, the default for others; 2 + v: variant v,
+ * 0..4); n, is_complex, precision and init are ignored (complex iff im != NULL,
+ * FP64, seeded random start).  `problems` is a HOST array.  Host outputs:
+ * eig_re / eig_im / residuals (count x wanted, row i = problem i in sort
  * order), status (count, oapb_status per problem).  Synchronises `stream`.
  * Returns OAPB_OK when every problem converged, OAPB_NOT_CONVERGED when some
  * did not (see status), or an error. */

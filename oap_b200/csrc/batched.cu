@@ -670,11 +670,15 @@ void remember_variant(const BatchKey& key, int v) {
 // Time the variants that can win on an evenly strided sample of the
 // size-sorted batch (two waves of the 256 x 2 grid: a sample of one problem per
 // SM hides what more resident CTAs give, and picked 256 x 1, 40.0 ms on 2048
-// problems that 256 x 2 solves in 31.5) with CUDA events; the sample's outputs
-// land in the batch's output slots and are overwritten by the full launch that
-// follows.  256 x 1 and 64 x 8 (its registers in local memory) lose on every
-// batch of more problems than SMs.  dsample: device room for the sample's
-// descriptors.
+// problems of 32..512 rows that 256 x 2 solves in 31.5) with CUDA events; the
+// sample's outputs land in the batch's output slots and are overwritten by the
+// full launch that follows.  256 x 2 wins while two problems of a batch fit an
+// SM's cache and registers; 256 x 1 where shared memory leaves one CTA per SM
+// to every variant (200 real problems of 1500..2048 rows, hdim 12: 33 ms, 256 x 2
+// 61) and on complex problems of 700..1024 rows at hdim 24 (200: 22 and 46 ms,
+// 1500: 143 and 197).  64 x 8 (its registers in local memory) is not timed: up to
+// four times the best, and under 10 % ahead only on 2000 problems of 16..48
+// rows at hdim 12.  dsample: device room for the sample's descriptors.
 int tune_batched(BatchArgs A, const std::vector<BatchDesc>& d, const int* grids, size_t smem, cudaStream_t s,
                  char* dsample, int* best) {
   const int count = (int)d.size();
@@ -694,7 +698,7 @@ int tune_batched(BatchArgs A, const std::vector<BatchDesc>& d, const int* grids,
   int rc = OAPB_OK;
   float best_ms = 0;
   *best = 2;
-  for (const int v : {2, 1, 3}) {
+  for (const int v : {2, 0, 1, 3}) {
     if (rc) break;
     if (cudaMemsetAsync((void*)A.counter, 0, 4 * sizeof(unsigned long long), s) != cudaSuccess ||
         cudaEventRecord(e0, s) != cudaSuccess ||
@@ -816,9 +820,9 @@ int oapb_arnoldi_solve_batched(const oapb_arnoldi_config* cfg, const oapb_batch_
       variant = cfg->autotune - 2;
     } else if (cfg->autotune == 1 && (int)count > kNumSMs) {
       // at most one problem per SM leaves 256 x 1, the default, untimed: there is
-      // no second problem to overlap with and no reason to give up registers
-      // (132 complex problems up to 413 rows: 2.65 ms, 256 x 2 3.25, the others
-      // 4.3 and more).
+      // no second problem to overlap with (132 complex problems up to 413 rows:
+      // 2.65 ms, 256 x 2 3.25, the others 4.3 and more; 64 to 140 problems from
+      // 16..48 to 300..512 rows: within 10 % of the best).
       // (sizes of like batches: the largest n to 64, the problems to a power of two)
       int cl = 0;
       while ((count >> cl) > 1 && cl < 12) ++cl;
