@@ -36,6 +36,7 @@
 #include <math.h>
 
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -341,6 +342,7 @@ struct oapb_mlp {
   std::vector<int> act;                // activation of each layer's outputs (oapb_activation)
   // activations for the last forward (capacity batch)
   int cap = 0;
+  void* acts = nullptr;                // the buffers below
   std::vector<float*> hf;              // FP32 activations per layer output (nl)
   std::vector<float*> zf;              // FP32 pre-activations per layer output (nl)
   std::vector<__nv_bfloat16*> hb;      // BF16 activations: input + per layer (rows padded)
@@ -351,54 +353,52 @@ struct oapb_mlp {
 
 namespace {
 
-int g_mlp_free_acts(oapb_mlp* h) {
-  for (auto p : h->hf) cudaFree(p);
-  for (auto p : h->hb) cudaFree(p);
-  for (auto p : h->zf) cudaFree(p);
-  h->hf.clear();
-  h->hb.clear();
-  h->zf.clear();
-  for (int i = 0; i < 2; ++i) {
-    if (h->dA[i]) cudaFree(h->dA[i]);
-    if (h->dAb[i]) cudaFree(h->dAb[i]);
-    h->dA[i] = nullptr;
-    h->dAb[i] = nullptr;
-  }
+void free_acts(oapb_mlp* h) {
+  if (h->acts) cudaFree(h->acts);
+  h->acts = nullptr;
   h->cap = 0;
-  return OAPB_OK;
 }
 
-// zeroed (the row pads stay zero)
-template <typename P>
-int zalloc(P** p, size_t bytes, cudaStream_t s) {
-  if (cudaMalloc(p, bytes) != cudaSuccess) {
-    *p = nullptr;
-    cudaGetLastError();
-    return OAPB_ERR_NOMEM;
-  }
-  return cudaMemsetAsync(*p, 0, bytes, s) == cudaSuccess ? OAPB_OK : OAPB_ERR_CUDA;
-}
-
+// The buffers of a batch, one allocation, zeroed: the row pads stay zero.
+// (Fourteen allocations with a fill each took most of a new network's first
+// step: 16 - 256 - 256 - 2056 at 256 samples 2.3 ms, 0.6 with one.)
 int ensure_acts(oapb_mlp* h, int batch, cudaStream_t s) {
   if (batch <= h->cap) return OAPB_OK;
-  g_mlp_free_acts(h);
+  free_acts(h);
   int mx = 0;
   for (int v : h->sz) mx = v > mx ? v : mx;
-  h->hb.resize(h->nl + 1, nullptr);
-  h->hf.resize(h->nl, nullptr);
-  h->zf.resize(h->nl, nullptr);
-  int rc = OAPB_OK;
-  for (int l = 0; l <= h->nl && !rc; ++l)
-    rc = zalloc(&h->hb[l], sizeof(__nv_bfloat16) * (size_t)batch * pad8(h->sz[l]), s);
-  for (int l = 0; l < h->nl && !rc; ++l) {
-    rc = zalloc(&h->hf[l], sizeof(float) * (size_t)batch * h->sz[l + 1], s);
-    if (!rc) rc = zalloc(&h->zf[l], sizeof(float) * (size_t)batch * h->sz[l + 1], s);
+  h->hb.assign(h->nl + 1, nullptr);
+  h->hf.assign(h->nl, nullptr);
+  h->zf.assign(h->nl, nullptr);
+  char* base = nullptr;
+  size_t total = 0;
+  for (int pass = 0; pass < 2; ++pass) {  // sizes, then addresses
+    size_t off = 0;
+    auto take = [&](auto** p, size_t values) {
+      if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + off);
+      off += (values * sizeof(**p) + 255) & ~(size_t)255;
+    };
+    const size_t b = (size_t)batch;
+    for (int l = 0; l <= h->nl; ++l) take(&h->hb[l], b * pad8(h->sz[l]));
+    for (int l = 0; l < h->nl; ++l) {
+      take(&h->hf[l], b * h->sz[l + 1]);
+      take(&h->zf[l], b * h->sz[l + 1]);
+    }
+    for (int i = 0; i < 2; ++i) {
+      take(&h->dA[i], b * mx);
+      take(&h->dAb[i], b * pad8(mx));
+    }
+    if (pass == 0) {
+      total = off;
+      if (cudaMalloc(&h->acts, total) != cudaSuccess) {
+        h->acts = nullptr;
+        cudaGetLastError();
+        return OAPB_ERR_NOMEM;
+      }
+      base = (char*)h->acts;
+    }
   }
-  for (int i = 0; i < 2 && !rc; ++i) {
-    rc = zalloc(&h->dA[i], sizeof(float) * (size_t)batch * mx, s);
-    if (!rc) rc = zalloc(&h->dAb[i], sizeof(__nv_bfloat16) * (size_t)batch * pad8(mx), s);
-  }
-  if (rc) return rc;
+  if (cudaMemsetAsync(h->acts, 0, total, s) != cudaSuccess) return OAPB_ERR_CUDA;
   h->cap = batch;
   return OAPB_OK;
 }
@@ -530,7 +530,7 @@ int oapb_mlp_create(oapb_mlp** out, const uint32_t* sizes, uint32_t nlayers, uin
 int oapb_mlp_destroy(oapb_mlp* h) {
   if (!h) return OAPB_ERR_ARG;
   cudaDeviceSynchronize();
-  g_mlp_free_acts(h);
+  free_acts(h);
   cudaFree(h->w);
   cudaFree(h->g);
   cudaFree(h->m1);
