@@ -222,7 +222,11 @@ typedef struct oapb_arnoldi_config {
   int32_t init;            /* oapb_init */
   uint32_t max_restarts;   /* restart budget (reference: CHECK_* rules) */
   double tolerance;        /* ||A x - l x|| / (|l_1| ||x||) goal, e.g. 1e-10 */
-  double rho;              /* DGKS threshold (CuHArnoldi::setRho, default 1/3.14) */
+  double rho;              /* DGKS threshold (CuHArnoldi::setRho, default 1/3.14);
+                              the implicit Gram operators take the second pass
+                              at every step whatever it is, and the first two
+                              steps after a restart of a symmetric operator
+                              take at least 1 */
   uint64_t seed;           /* start-vector seed for OAPB_INIT_RANDOM */
   int32_t profile;         /* 1: time every dense matvec with CUDA events
                               (oapb_arnoldi_stats.matvec_seconds) */
@@ -288,8 +292,8 @@ typedef struct oapb_arnoldi_stats {
   double pass_kernel_seconds[3];
   uint32_t pass_kernel_timed[3];
   uint32_t symtri;           /* restart-loop eigensolves of the last plain solve
-                                that took the Hermitian tridiagonal path
-                                (Hermitian or real symmetric operators) */
+                                that took the symmetric path (Hermitian or real
+                                symmetric operators) */
 } oapb_arnoldi_stats;
 
 typedef struct oapb_arnoldi oapb_arnoldi;   /* opaque solver handle */
@@ -315,11 +319,11 @@ OAPB_EXPORT int oapb_arnoldi_set_callback(oapb_arnoldi* handle, oapb_matvec_fn f
 
 /* Implicit Gram operator A = X X^T for FP32 images X (rows = n samples x
  * cols pixels, row-major, device; 16-byte aligned when cols % 4 == 0):
- * every operator application runs w = X (X^T v) in two HBM-bound passes
- * over X, FP64 accumulation, without forming A (the reference application
- * rebuilds the Gram on every multiplication, oap2dt3dDevice/
- * MainAPExecutor.cpp:42-127, SquareMatrixApi.cpp:143-181).  Real solves
- * only; runs the FP64 path.  X must stay valid during solves. */
+ * every operator application runs w = X (X^T v), FP64 accumulation, in one
+ * pass over X (up to 8192 rows and X 16-byte aligned, else two), without
+ * forming A (the reference application rebuilds the Gram on every
+ * multiplication, oap2dt3dDevice/MainAPExecutor.cpp:42-127,
+ * SquareMatrixApi.cpp:143-181).  Real solves only; runs the FP64 path.  X must stay valid during solves. */
 OAPB_EXPORT int oapb_arnoldi_set_gram_operator(oapb_arnoldi* handle, const float* X, uint32_t rows,
                                                uint32_t cols);
 

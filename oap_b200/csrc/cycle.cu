@@ -21,9 +21,9 @@
 // are not 16-byte aligned).  A warp takes a pair of rows times a column
 // segment; the segment count evens the pairs out over the 16 warps.
 //
-// Measured (B200, whole step): real n = 2048, m = 24: 50 us on the per-step
-// kernels, 14.9 us here; complex n = 3001, m = 32: 105 us, 37 us; complex
-// n = 6000, m = 48 (576 MB per pass, HBM-bound): 140 us, 110 us.
+// Measured (B200, whole step): real n = 2048, m = 24: 35 us on the per-step
+// kernels, 13.4 us here; complex n = 3001, m = 32: 93 us, 37 us; complex
+// n = 6000, m = 48 (576 MB per pass, HBM-bound): 169 us, 101 us.
 //
 // Every wait is bounded (2 s): a barrier that runs out sets bit 1 of
 // DevState::status and the CTA returns.

@@ -4,9 +4,9 @@
 // X X^T, or row blocks of it, on every multiplication through
 // SquareMatrixApi::getDeviceMatrix / getDeviceSubMatrix,
 // oapMatrixCuda/SquareMatrixApi.cpp:143-181).  Here A is never formed, and one
-// application reads X once (k_gram_fused): a thread-block cluster holds a panel
-// of 8 to 64 columns of all rows in its CTAs' shared memory, forms the panel's
-// t = X_p^T v (the CTAs' sums exchanged through distributed shared memory) and
+// application reads X once (k_gram_fused): a thread-block cluster copies a panel
+// of 8 to 64 columns of all rows through shared memory into its CTAs' registers,
+// forms the panel's t = X_p^T v (the CTAs' sums exchanged through distributed shared memory) and
 // adds X_p t to its rows' sums, which stay in registers over all its panels.
 // Above 8192 rows, beyond a cluster, and for X that is not 16-byte aligned, two
 // passes over X:
@@ -23,7 +23,7 @@
 // A v = sum_c X_c (X_c^T v), so one application reads X exactly once.  The
 // first blocks that fit the caller's device budget stay resident; the rest
 // stream through two device buffers, the host-to-device copy of the next
-// block (on its own stream) overlapping the two passes over the current one.
+// block (on its own stream) overlapping the application of the current one.
 #include <algorithm>
 #include <map>
 #include <mutex>

@@ -706,9 +706,10 @@ int arnoldi_step(oapb_arnoldi* a, int j, bool fp32) {
   if ((rc = gs_pass<C>(a, j, a->wre, a->wim, a->h, 0))) return rc;
   ++a->stats.kernel_launches;
   // A Gram operator's application reads X (hundreds of microseconds at the
-  // sizes it is for), so its vectors are reorthogonalised at every step: the
-  // rho rule leaves 1e-6 of orthogonality on image spectra, and H then fails
-  // the symmetry check (a general eigensolve at m = 96 took 20 ms)
+  // sizes it is for), so its vectors are reorthogonalised at every step, whatever
+  // cfg.rho (the header says so): the rho rule leaves 1e-6 of orthogonality on
+  // image spectra, and H then fails the symmetry check (a general eigensolve at
+  // m = 96 took 20 ms)
   const double rho = (a->gX || a->gS) ? 1e300 : a->cfg.rho;
   launch_dependent(k_gs_finalize, dim3(1), dim3(256), 0, s, a->fpart, a->nupd, a->h, a->s, a->H, m, j, rho, a->st, 0,
                    !C);

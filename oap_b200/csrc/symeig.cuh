@@ -137,11 +137,12 @@ __device__ __forceinline__ void sym_z(double* Z, int m, int ld, int M, int r, co
 // eigenvectors; false when the sweeps ran out.  All nthr threads of the CTA.
 //
 // A round's time is latency: one rotation's arithmetic, the block update and
-// two barriers (m = 24: 154 us per check with an FP64 rotation and A and Z on
-// the same threads, 90 us here; m = 32: 237 and 144 us).  For m <= 32 on 512 threads one half updates A and the other
-// Z.  Tried and not kept: every thread forming the two rotations of its block
-// itself, with one barrier per round and two copies of A (112 against 98 us
-// at m = 24, 182 against 152 us at m = 32: the repeated FP64 arithmetic).
+// two barriers (k_symeig, m = 24: 154 us with an FP64 rotation and A and Z on the
+// same threads, 90 us here; m = 32: 237 and 144 us).  For m <= 32 on 512 threads
+// one half updates A and the other Z.  Tried and not kept: every thread forming
+// the two rotations of its block itself, with one barrier per round and two copies
+// of A (a seventh slower at m = 24, a fifth at m = 32: the repeated FP64
+// arithmetic).
 static __device__ bool cta_jacobi(double* A, double* Z, int m, int ld, const SymScratch& S, int tid, int nthr) {
   const int M = sym_even(m), h = M / 2;
   const bool split = h <= 16 && nthr >= 512;
