@@ -229,7 +229,11 @@ static __device__ bool sym_eig(const HessArgs& a, double* A, double* Z, const Sy
     return true;
   }
   for (int i = tid; i < m; i += nthr) {
-    const double kv = sort_key(cplx{A[i + i * ld], 0}, a.which);
+    // (the imaginary parts all tie: the largest |value| first, which a restarted
+    // space finds; in diagonal order the wanted set was an arbitrary one inside
+    // the spectrum, another after every restart, and the loop did not converge)
+    const bool ties = a.which == OAPB_SORT_LARGEST_IM || a.which == OAPB_SORT_SMALLEST_IM;
+    const double kv = ties ? -fabs(A[i + i * ld]) : sort_key(cplx{A[i + i * ld], 0}, a.which);
     S.key[i] = (kv != kv) ? INFINITY : kv;
   }
   __syncthreads();
