@@ -475,9 +475,13 @@ __device__ void solve_one(const BatchArgs& A, const BatchDesc& P, int slot, cons
       h.use_beta = 1;
       h.tol = A.tol;
       h.beta = 0;
-      // a third of the way from k to m: fewer operator applications (4 of 24
-      // with 4 outlying values: 44 -> 38) for the same number of restarts
-      h.keep = k + (m - k) / 3 < m ? k + (m - k) / 3 : k;
+      // a third of the way from k to m where that leaves enough steps per
+      // restart: fewer operator applications (4 of 24 with 4 outlying values:
+      // 44 -> 38) for the same number of restarts.  Up to k + 10 vectors the
+      // shorter cycles need more restarts on spectra without a gap (24 normal
+      // matrices of 80 to 150 rows, 6 wanted: m = k + 5 1211 with the wanted
+      // alone and 2163, m = k + 10 254 and 315): the wanted alone
+      h.keep = m - k > 10 ? k + (m - k) / 3 : k;
       h.keep_sym = restart_keep(m, k, true);
       // a symmetric H on the whole CTA, any other on two warps.  Q is written
       // only at the end of hess_core: until then it is the rotation list and

@@ -68,10 +68,14 @@ struct HessArgs {
 // Vectors a restart keeps on the symmetric path: one guard vector beyond the
 // wanted.  It takes most of what more would give (over 32 operators with 8 of
 // 24 at a spectrum's edge, 7800 applications with none, 5600 with one, 4600
-// with five; more of them also leave a warm start little to save).  On the
-// general path a restart costs as much as 10 - 30 applications (its Schur
-// form), and more kept vectors mean more restarts: the wanted alone.
-__host__ __device__ inline int restart_keep(int m, int k, bool sym) { return sym && k + 1 < m ? k + 1 : k; }
+// with five; more of them also leave a warm start little to save).  In a space
+// of fewer than k + 4 vectors it takes too much of what a restart adds (24 Gaussian
+// symmetric operators of 80 to 150 rows, one wanted: m = k + 2 4017 restarts in
+// all without it and 7266 with it, k + 3 1892 and 1982, k + 4 1116 and 971, k + 5
+// 752 and 594).  On the general path a restart costs as much as 10 - 30
+// applications (its Schur form), and more kept vectors mean more restarts: the
+// wanted alone.
+__host__ __device__ inline int restart_keep(int m, int k, bool sym) { return sym && m - k >= 4 ? k + 1 : k; }
 
 // leading dimension of the T / Z work arrays (odd)
 __host__ __device__ __forceinline__ int hess_ld(int m) { return m | 1; }
