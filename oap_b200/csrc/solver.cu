@@ -786,9 +786,18 @@ int read_state(oapb_arnoldi* a, DevState* h) {
 // vector does not fit a CTA's shared memory (n above about 10000 complex /
 // 20000 real, where the operator pass takes 90 % of a step), and where a
 // caller asks for the launches themselves: a forced variant of the operator
-// pass or the event timing of every pass.
+// pass or the event timing of every pass.  The chosen form of a small operator
+// has no such pass and runs in cycles with either (n = 82, 5 restarts: 1.0 ms,
+// 2.1 on the per-step kernels).
+constexpr int kOnchipMaxN = 2048;
+constexpr int kOnchipMaxM = 32;
+bool small_chosen(const oapb_arnoldi* a) {
+  return a->cfg.precision == OAPB_PREC_MIXED && a->n <= kOnchipMaxN && a->m <= kOnchipMaxM &&
+         a->cfg.init == OAPB_INIT_RANDOM && a->start_shifts.empty();
+}
 bool use_cycle(const oapb_arnoldi* a) {
-  return a->have_cycle && !a->cb && !a->gX && !a->gS && a->a64re && !a->cfg.profile && a->cfg.autotune < 2;
+  return a->have_cycle && !a->cb && !a->gX && !a->gS && a->a64re &&
+         (small_chosen(a) || (!a->cfg.profile && a->cfg.autotune < 2));
 }
 
 // Two cooperative grids that each held part of the SMs would wait for one
@@ -1255,10 +1264,6 @@ int ensure_side_stream(oapb_arnoldi* a) {
 
 constexpr int kSlow = 100;   // subspace(): convergence too slow for the iteration budget
 constexpr int kMixedMinN = 8192;
-// The chosen form for small dense operators is the FP64 restart loop (one
-// launch per cycle); the stats report it up to these sizes.
-constexpr int kOnchipMaxN = 2048;
-constexpr int kOnchipMaxM = 32;
 // BF16 operator passes (tensor cores only).  In the FP32-class subspace
 // iteration: the powers taken while the block is still far from the wanted
 // subspace (before the first check, then while the residual extrapolated
@@ -1825,8 +1830,7 @@ int solve_impl(oapb_arnoldi* a, double* eig_re, double* eig_im, double* res, boo
   a->ckpt_ready = false;
   // (the chosen form of a small dense operator: the basis and, where it fits,
   // the operator stay in shared memory through each restart cycle)
-  a->stats.onchip = !resume && !mixed && a->cfg.precision == OAPB_PREC_MIXED && use_cycle(a) && a->n <= kOnchipMaxN &&
-                    a->m <= kOnchipMaxM && a->cfg.init == OAPB_INIT_RANDOM && a->start_shifts.empty();
+  a->stats.onchip = !resume && small_chosen(a) && use_cycle(a);
   int st = resume ? resume_plain<C>(a, r.data())
            : mixed ? solve_mixed<C>(a, r.data())
                     : solve_plain<C>(a, r.data());
