@@ -178,7 +178,9 @@ OAPB_EXPORT int oapb_selftest_gram_wait(uint32_t limit_us, int32_t late, int32_t
 /* Solver: CuHArnoldi / CuHArnoldiCallback (ArnoldiPackage)                  */
 /* ------------------------------------------------------------------------ */
 
-/* Wanted-set ordering, ArnUtils::Sort* (ArnoldiPackage/ArnoldiUtils.cpp:24-50). */
+/* Wanted-set ordering, ArnUtils::Sort* (ArnoldiPackage/ArnoldiUtils.cpp:24-50).
+ * The orders by imaginary part tie on a symmetric or Hermitian operator: values of
+ * largest magnitude first. */
 typedef enum oapb_sort {
   OAPB_SORT_LARGEST_VALUES = 0,     /* |lambda| descending (LM) */
   OAPB_SORT_LARGEST_RE = 1,
