@@ -179,8 +179,9 @@ OAPB_EXPORT int oapb_selftest_gram_wait(uint32_t limit_us, int32_t late, int32_t
 /* ------------------------------------------------------------------------ */
 
 /* Wanted-set ordering, ArnUtils::Sort* (ArnoldiPackage/ArnoldiUtils.cpp:24-50).
- * The orders by imaginary part tie on a symmetric or Hermitian operator: values of
- * largest magnitude first. */
+ * The orders by imaginary part tie on a symmetric or Hermitian operator: up to
+ * hdim = 118 the values of largest magnitude come first, beyond it no order among
+ * them is promised. */
 typedef enum oapb_sort {
   OAPB_SORT_LARGEST_VALUES = 0,     /* |lambda| descending (LM) */
   OAPB_SORT_LARGEST_RE = 1,
