@@ -39,6 +39,6 @@ def test_tuned_variant_is_among_the_fastest(count, lo, hi, cplx, hdim, k):
         return min(out[1:])
 
     tuned = best(True)
-    # the variants are up to a factor of two and more apart here; a quarter
-    # covers the noise of a timed sample
-    assert tuned <= 1.25 * min(best(2 + v) for v in range(5))
+    # every variant but the fastest takes 1.7 times its time and more here; half
+    # of it covers the noise of a timed sample and of the host
+    assert tuned <= 1.5 * min(best(2 + v) for v in range(5))
